@@ -57,7 +57,10 @@ __global__ void __launch_bounds__(256) pack_boards_kernel(unsigned long long flo
     }
     __syncthreads();
     for (int p = tid; p < kHands; p += blockDim.x) {
-        if (seen[p] != 1) atomicOr(&bad, 2);
+        if (seen[p] != 1) {  // no hand, or two: sorted[p] is not to be used as an index
+            atomicOr(&bad, 2);
+            continue;
+        }
         int h = sorted[p];
         int hc1 = cards_of[h] & 255, hc2 = cards_of[h] >> 8;
         bool blocked = ((1ull << hc1) | (1ull << hc2)) & board;
