@@ -117,6 +117,7 @@ bool river_tree_matches() {
 constexpr int kPipeChunks = 4;  // chunks of a staged pass (copies overlap the kernel)
 
 struct Builder {
+    RiverScratch scratch;  // of passes over few roots
     std::vector<SubgameDesc> desc;
     int capacity = 0;
     float *comm = nullptr;  // pinned staging, capacity rows of kRangeStride
@@ -332,7 +333,7 @@ int evaluate_impl(Builder *b, EvalTables *t, int player, int exploit, const floa
             e = launch_river(exploit ? kModeBR : kModeCFR, b->d_desc + lo, hi - lo, b->d_ranges + row0,
                              b->d_results + row0, b->d_regrets + (size_t)lo * kEdges * kBuckets, t->packs, t->flop,
                              player, t->max_groups, t->max_card_groups, avg ? b->d_own + row0 : nullptr,
-                             avg ? b->d_avg + (size_t)lo * kEdges * kBuckets : nullptr, s);
+                             avg ? b->d_avg + (size_t)lo * kEdges * kBuckets : nullptr, &b->scratch, s);
             if (e != cudaSuccess) return fail(kErrCuda, "river kernel launch", e);
             if ((e = cudaEventRecord(b->ev_done[k], s)) != cudaSuccess ||
                 (e = cudaStreamWaitEvent(b->copy_out, b->ev_done[k], 0)) != cudaSuccess)
@@ -355,7 +356,7 @@ int evaluate_impl(Builder *b, EvalTables *t, int player, int exploit, const floa
     }
     e = launch_river(exploit ? kModeBR : kModeCFR, b->d_desc, n, d_in, d_out, b->d_regrets, t->packs,
                      t->flop, player, t->max_groups, t->max_card_groups, avg ? (staged ? b->d_own : d_own) : nullptr,
-                     avg ? b->d_avg : nullptr, s);
+                     avg ? b->d_avg : nullptr, &b->scratch, s);
     if (e != cudaSuccess) return fail(kErrCuda, "river kernel launch", e);
     if (staged) {
         e = cudaMemcpyAsync(b->comm, b->d_results, (size_t)n * kRangeStride * sizeof(float),
@@ -888,7 +889,7 @@ int br64_impl(Builder *b, EvalTables *t, int updating_player, const double *rang
     cudaError_t e;
     if (!staged) {
         e = launch_river_br64(b->d_desc, n, ranges, results, b->d_regrets, t->packs, t->flop, updating_player,
-                              t->max_groups, t->max_card_groups, stream ? stream : b->stream);
+                              t->max_groups, t->max_card_groups, &b->scratch, stream ? stream : b->stream);
         return e == cudaSuccess ? kOk : fail(kErrCuda, "double best-response launch", e);
     }
     if (b->cap64 < b->dev_capacity) {
@@ -908,7 +909,7 @@ int br64_impl(Builder *b, EvalTables *t, int updating_player, const double *rang
                           kHands * sizeof(double), n, cudaMemcpyHostToDevice, b->stream);
     if (e != cudaSuccess) return fail(kErrCuda, "double range upload", e);
     e = launch_river_br64(b->d_desc, n, b->d_ranges64, b->d_results64, b->d_regrets, t->packs, t->flop,
-                          updating_player, t->max_groups, t->max_card_groups, b->stream);
+                          updating_player, t->max_groups, t->max_card_groups, &b->scratch, b->stream);
     if (e != cudaSuccess) return fail(kErrCuda, "double best-response launch", e);
     e = cudaMemcpy2DAsync(results, kHands * sizeof(double), b->d_results64, kRangeStride * sizeof(double),
                           kHands * sizeof(double), n, cudaMemcpyDeviceToHost, b->stream);

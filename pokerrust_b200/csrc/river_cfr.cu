@@ -45,6 +45,7 @@ namespace prb {
 
 namespace {
 
+constexpr int kMaxSplitRoots = 240;    // roots of a pass whose river cards may be split over CTAs
 constexpr int NT = 512;                // threads per CTA
 constexpr int kGPer = 9;               // warps 0-3: rank list slots per lane (128 * 9 >= 1082)
 constexpr int kCPer = 6;               // card list slots per lane (8 lanes * 6 = 48)
@@ -172,6 +173,18 @@ struct Smem {
           scale(reinterpret_cast<float *>(base + L.scale)),
           stage(reinterpret_cast<float(*)[2][ACC]>(base + L.stage)),
           stage_key(reinterpret_cast<int(*)[2]>(base + L.stage_key)) {}
+};
+
+// What a CTA of a split pass leaves behind per river card (launch_river: few roots, the river cards of
+// a root spread over CTAs): the bucket sums of that card as the one-CTA pass adds them to its
+// accumulators, so that finish_kernel can add them in the same order.
+template <int ACC>
+struct RiverPart {
+    alignas(16) float first[kBuckets][ACC];  // the first (and mostly only) sum of a bucket, 0 if it has none
+    float stage[2 * kOutWarps][ACC];      // runs touching an output warp's ends
+    float total[kNumLeaves];              // opponent weight of each leaf
+    int stage_key[2 * kOutWarps];
+    uint8_t next[kBuckets], last[kBuckets];  // second and last staged run of a bucket (255, 0: none)
 };
 
 __device__ __forceinline__ void bar_rank_list() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
@@ -311,12 +324,92 @@ __device__ __forceinline__ V vmax(V a, V b) {
     return a > b ? a : b;
 }
 
-template <int MODE, typename V, bool AVG, int UPD>
+__device__ __forceinline__ void load_regrets(int b, const float *greg, float (&reg)[kEdges]) {
+#pragma unroll
+    for (int e = 0; e < kEdges; e++) reg[e] = greg[e * kBuckets + b];
+}
+
+// Update of bucket b's regrets `reg`, once per subgame and pass (poker.cu:450-487,524-574), from its
+// leaf sums (and own-range mass) over the rivers.
+template <bool AVG>
+__device__ __forceinline__ void update_bucket(int b, float (&reg)[kEdges], const float *sums, const float *scale,
+                                              int updater, float *greg, float *gavg) {
+    if constexpr (AVG) {
+        // average-strategy sums: own range mass of the bucket over the rivers, times the
+        // updater's reach into the state, times the action probability (current regrets)
+        float reach[kStates];
+        reach[1] = sums[kNumLeaves];
+#pragma unroll
+        for (int di = 0; di < kNumDecision; di++) {
+            const int s = kDecision(di);
+            const int nk = kNChild(s);
+            float sum = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (k < nk) sum += reg[kEdge(s, k)];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if (k < nk) {
+                    const float sig = sum <= 1e-4f ? 1.0f / (float)nk : reg[kEdge(s, k)] / sum;
+                    const int c = kChild(s, k);
+                    reach[c] = kActor(s) == updater ? __fmul_rn(reach[s], sig) : reach[s];
+                    if (kActor(s) == updater) {
+                        float &sum_at = gavg[kEdge(s, k) * kBuckets + b];
+                        sum_at = kNChild(c) > 0 ? __fadd_rn(sum_at, reach[c]) : __fmaf_rn(reach[s], sig, sum_at);
+                    }
+                }
+            }
+        }
+    }
+    // which products are rounded together with their sums is fixed here, so that the whole and the
+    // split pass agree to the last bit
+    float A[kStates];
+#pragma unroll
+    for (int Lf = 0; Lf < kNumLeaves; Lf++) A[kLeaf(Lf)] = __fmul_rn(sums[Lf], scale[Lf]);
+#pragma unroll
+    for (int di = kNumDecision - 1; di >= 0; di--) {
+        const int s = kDecision(di);
+        const int nk = kNChild(s);
+        if (kActor(s) == updater) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (k < nk) sum += reg[kEdge(s, k)];
+            float node = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if (k < nk) {
+                    const float sig = sum <= 1e-4f ? 1.0f / (float)nk : reg[kEdge(s, k)] / sum;
+                    node = __fmaf_rn(sig, A[kChild(s, k)], node);
+                }
+            }
+            A[s] = node;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if (k < nk) {
+                    const int e = kEdge(s, k);
+                    reg[e] = fmaxf(__fadd_rn(reg[e], __fsub_rn(A[kChild(s, k)], node)), 0.0f);
+                    greg[e * kBuckets + b] = reg[e];
+                }
+            }
+        } else {
+            float node = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (k < nk) node = __fadd_rn(node, A[kChild(s, k)]);
+            A[s] = node;
+        }
+    }
+}
+
+// SPLIT: `splits` CTAs share a root, each with 48 / splits of its river cards, and leave their sums to
+// finish_kernel: the values in outs [root][split][hand], the bucket sums in parts [root][river card].
+template <int MODE, typename V, bool AVG, int UPD, bool SPLIT>
 __global__ void __launch_bounds__(NT, 1)
     river_kernel(const SubgameDesc *__restrict__ desc, const V *__restrict__ ranges, V *__restrict__ results,
                  float *__restrict__ regrets, const BoardPack *__restrict__ packs, unsigned long long flop,
                  int updater, int max_groups, int max_card_groups, const float *__restrict__ own_ranges,
-                 float *__restrict__ avg_sums) {
+                 float *__restrict__ avg_sums, int splits, V *__restrict__ outs, void *__restrict__ parts) {
     static_assert(MODE == kModeBR || sizeof(V) == 4, "CFR runs in single precision");
     static_assert(!AVG || MODE == kModeCFR, "average strategies accumulate in CFR passes");
     constexpr int ACC = kNumLeaves + (AVG ? 1 : 0);
@@ -326,10 +419,12 @@ __global__ void __launch_bounds__(NT, 1)
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int sg = blockIdx.x;
+    const int sg = SPLIT ? blockIdx.x / splits : blockIdx.x;
     const SubgameDesc d = desc[sg];
     const float bet = d.bet;
     float *greg = regrets + (size_t)sg * kEdges * kBuckets;
+
+    if constexpr (SPLIT) asm volatile("griddepcontrol.launch_dependents;");  // finish_kernel may get in place
 
     // ---- subgame setup: range, per-bucket reach tables ----
     for (int i = tid; i < kRangeStride; i += NT) {
@@ -396,15 +491,20 @@ __global__ void __launch_bounds__(NT, 1)
     __syncthreads();
 
     // ---- the 48 river cards ----
-    int rc_done = 0;
+    const int per_cta = SPLIT ? 48 / splits : 48;
+    const int first_river = SPLIT ? blockIdx.x % splits * per_cta : 0;
+    int rc_done = 0, nth = -1;
     for (int rc = 0; rc < 52; rc++) {
         const unsigned long long rb = 1ull << rc;
         if (rb & d.board4) continue;
+        nth++;
+        if (SPLIT && (nth < first_river || nth >= first_river + per_cta)) continue;
+        RiverPart<ACC> *part = SPLIT && MODE == kModeCFR ? static_cast<RiverPart<ACC> *>(parts) + (size_t)sg * 48 + nth : nullptr;
         const int slot = pair_index((d.board4 | rb) ^ flop);
         const BoardPack *__restrict__ pk = packs + slot;
         __syncthreads();  // previous river's readers are done with Pg, VC, Cf, Tf
         if constexpr (MODE == kModeCFR) {
-            if (warp == NT / 32 - 1 && lane < ACC && rc_done > 0) resolve_stage(S, lane);
+            if (!SPLIT && warp == NT / 32 - 1 && lane < ACC && rc_done > 0) resolve_stage(S, lane);
         }
         rc_done++;
 
@@ -482,8 +582,11 @@ __global__ void __launch_bounds__(NT, 1)
                 if constexpr (MODE == kModeCFR) {
                     // blocked hands' contribution to bucket 0 (see the file comment)
 #pragma unroll
-                    for (int c = 0; c < kNumLeaves; c++)
-                        S.abar[0][c] += (c < kNumSD ? -235.0f : 235.0f) * total[leaf_channel(c, UPD)];
+                    for (int c = 0; c < kNumLeaves; c++) {
+                        const float t = total[leaf_channel(c, UPD)];
+                        if constexpr (SPLIT) part->total[c] = t;
+                        else S.abar[0][c] = __fmaf_rn(c < kNumSD ? -235.0f : 235.0f, t, S.abar[0][c]);
+                    }
                 }
             }
             // W - B of every tie group: prefix at its start + prefix at its end - total
@@ -738,8 +841,44 @@ __global__ void __launch_bounds__(NT, 1)
                 }
             }
         }
+        if constexpr (SPLIT && MODE == kModeCFR) {
+            // this river card's bucket sums leave; the accumulators start at zero for the next one
+            __syncthreads();
+            const int *key = &S.stage_key[0][0];
+            const float *stage = &S.stage[0][0][0];
+            uint8_t *first = reinterpret_cast<uint8_t *>(S.Pg);  // first staged run of each bucket
+            if (tid < kBuckets) {
+                int from = 255, next = 255, last = 0;
+                for (int i = 0; i < kOutWarps * 2; i++) {
+                    if (key[i] != tid) continue;
+                    if (from == 255) from = i;
+                    else if (next == 255) next = i;
+                    last = i;
+                }
+                first[tid] = (uint8_t)from;
+                part->next[tid] = (uint8_t)next;
+                part->last[tid] = (uint8_t)last;
+            }
+            __syncthreads();
+            if (tid < kOutWarps * 2 * ACC) {
+                const int i = tid / ACC, c = tid % ACC;
+                (&part->stage[0][0])[tid] = stage[tid];
+                if (c == 0) part->stage_key[i] = key[i];
+                if (key[i] >= 0 && first[key[i]] == i) S.abar[key[i]][c] = stage[tid];  // no other sum is there
+            }
+            __syncthreads();
+            float4 *abar = reinterpret_cast<float4 *>(&S.abar[0][0]), *to = reinterpret_cast<float4 *>(&part->first[0][0]);
+            for (int i = tid; i < kBuckets * ACC / 4; i += NT) {
+                to[i] = abar[i];
+                abar[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        }
     }
     __syncthreads();
+    if constexpr (SPLIT) {
+        for (int i = tid; i < kRangeStride; i += NT) outs[(size_t)blockIdx.x * kRangeStride + i] = S.out[i];
+        return;
+    }
     if constexpr (MODE == kModeCFR) {
         if (warp == NT / 32 - 1 && lane < ACC) resolve_stage(S, lane);
         __syncthreads();
@@ -752,106 +891,212 @@ __global__ void __launch_bounds__(NT, 1)
         for (int i = tid; i < kRangeStride; i += NT) dst[i] = i < kHands ? S.out[i] * inv : V(0);
     }
 
-    // ---- regret update, once per subgame (poker.cu:450-487,524-574) ----
     if constexpr (MODE == kModeCFR) {
         if (tid < kBuckets) {
-            const int b = tid;
             float reg[kEdges];
-#pragma unroll
-            for (int e = 0; e < kEdges; e++) reg[e] = greg[e * kBuckets + b];
-            if constexpr (AVG) {
-                // average-strategy sums: own range mass of the bucket over the rivers, times the
-                // updater's reach into the state, times the action probability (current regrets)
-                float reach[kStates];
-                reach[1] = S.abar[b][kNumLeaves];
-                float *gavg = avg_sums + (size_t)sg * kEdges * kBuckets;
-#pragma unroll
-                for (int di = 0; di < kNumDecision; di++) {
-                    const int s = kDecision(di);
-                    const int nk = kNChild(s);
-                    float sum = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < 3; k++)
-                        if (k < nk) sum += reg[kEdge(s, k)];
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        if (k < nk) {
-                            const float sig = sum <= 1e-4f ? 1.0f / (float)nk : reg[kEdge(s, k)] / sum;
-                            const int c = kChild(s, k);
-                            reach[c] = kActor(s) == updater ? reach[s] * sig : reach[s];
-                            if (kActor(s) == updater) gavg[kEdge(s, k) * kBuckets + b] += reach[s] * sig;
-                        }
-                    }
-                }
-            }
-            float A[kStates];
-#pragma unroll
-            for (int Lf = 0; Lf < kNumLeaves; Lf++) A[kLeaf(Lf)] = S.abar[b][Lf] * S.scale[Lf];
-#pragma unroll
-            for (int di = kNumDecision - 1; di >= 0; di--) {
-                const int s = kDecision(di);
-                const int nk = kNChild(s);
-                if (kActor(s) == updater) {
-                    float sum = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < 3; k++)
-                        if (k < nk) sum += reg[kEdge(s, k)];
-                    float node = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        if (k < nk) {
-                            const float sig = sum <= 1e-4f ? 1.0f / (float)nk : reg[kEdge(s, k)] / sum;
-                            node += sig * A[kChild(s, k)];
-                        }
-                    }
-                    A[s] = node;
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        if (k < nk) {
-                            const int e = kEdge(s, k);
-                            reg[e] = fmaxf(reg[e] + (A[kChild(s, k)] - node), 0.0f);
-                            greg[e * kBuckets + b] = reg[e];
-                        }
-                    }
-                } else {
-                    float node = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < 3; k++)
-                        if (k < nk) node += A[kChild(s, k)];
-                    A[s] = node;
-                }
-            }
+            load_regrets(tid, greg, reg);
+            update_bucket<AVG>(tid, reg, S.abar[tid], S.scale, updater, greg,
+                               AVG ? avg_sums + (size_t)sg * kEdges * kBuckets : nullptr);
         }
     }
 }
 
+// Second half of a split pass: adds up the river cards' parts of root blockIdx.x in the order of the
+// one-CTA pass, writes the results and updates the regrets; CTA y of a root takes kFinBuckets buckets
+// and a share of the hands. One thread per bucket and sum (the loads of a warp are consecutive); the
+// last warp, one thread per bucket, has the regrets in hand by the time the sums are there. It is
+// launched beside the pass's first half and waits for it (programmatic dependent launch).
+constexpr int kFinBuckets = 16;
+constexpr int kFinThreads = kFinBuckets * 18 + 32;
+template <int MODE, typename V, bool AVG, int UPD>
+__global__ void __launch_bounds__(kFinThreads)
+    finish_kernel(const SubgameDesc *__restrict__ desc, const V *__restrict__ outs, int splits,
+                  const void *__restrict__ parts, V *__restrict__ results, float *__restrict__ regrets,
+                  float *__restrict__ avg_sums) {
+    constexpr int ACC = kNumLeaves + (AVG ? 1 : 0);
+    const int sg = blockIdx.x, tid = threadIdx.x;
+    if constexpr (MODE == kModeCFR) {
+        __shared__ float sums[kFinBuckets][ACC], scale[kNumLeaves];
+        float *greg = regrets + (size_t)sg * kEdges * kBuckets;
+        if (tid >= kFinBuckets * 18) {
+            const int t = tid - kFinBuckets * 18, b = blockIdx.y * kFinBuckets + t;
+            if (t < kNumLeaves) scale[t] = leaf_scale(kLeaf(t), UPD, desc[sg].bet);
+            float reg[kEdges];
+            if (t < kFinBuckets) load_regrets(b, greg, reg);
+            asm volatile("bar.sync 1, %0;" ::"n"(kFinThreads) : "memory");
+            if (t < kFinBuckets)
+                update_bucket<AVG>(b, reg, sums[t], scale, UPD, greg,
+                                   AVG ? avg_sums + (size_t)sg * kEdges * kBuckets : nullptr);
+            return;
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const int c = tid % ACC, b = blockIdx.y * kFinBuckets + tid / ACC;
+        if (tid < kFinBuckets * ACC) {
+            const RiverPart<ACC> *p = static_cast<const RiverPart<ACC> *>(parts) + (size_t)sg * 48;
+            float acc = 0.0f;
+            constexpr int kAhead = 16;
+#pragma unroll 1
+            for (int k0 = 0; k0 < 48; k0 += kAhead) {
+                float first[kAhead], total[kAhead], second[kAhead];
+                int next[kAhead], last[kAhead];
+#pragma unroll
+                for (int q = 0; q < kAhead; q++) {
+                    first[q] = p[k0 + q].first[b][c];
+                    next[q] = p[k0 + q].next[b];
+                    last[q] = p[k0 + q].last[b];
+                    total[q] = b == 0 && c < kNumLeaves ? p[k0 + q].total[c] : 0.0f;
+                }
+#pragma unroll
+                for (int q = 0; q < kAhead; q++) second[q] = next[q] != 255 ? p[k0 + q].stage[next[q]][c] : 0.0f;
+#pragma unroll
+                for (int q = 0; q < kAhead; q++) {
+                    // blocked hands' contribution to bucket 0 (see the file comment)
+                    if (b == 0 && c < kNumLeaves) acc = __fmaf_rn(c < kNumSD ? -235.0f : 235.0f, total[q], acc);
+                    acc += first[q];
+                    acc += second[q];
+                    for (int i = next[q] + 1; i <= last[q]; i++)  // a bucket of more than two warps' hands
+                        if (p[k0 + q].stage_key[i] == b) acc += p[k0 + q].stage[i][c];
+                }
+            }
+            sums[tid / ACC][c] = acc;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kFinThreads) : "memory");
+    } else {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+    constexpr int kShare = kRangeStride / (kBuckets / kFinBuckets);
+    for (int i = tid; i < kShare; i += kFinBuckets * 18) {
+        const int h = blockIdx.y * kShare + i;
+        V sum = V(0);
+        for (int q = 0; q < splits; q++) sum += outs[((size_t)sg * splits + q) * kRangeStride + h];
+        results[(size_t)sg * kRangeStride + h] = h < kHands ? sum * (V(1) / V(48)) : V(0);
+    }
+}
+
+// CTAs per root. One CTA takes a root's 48 river cards one after the other, so few roots leave most
+// of the chip idle; more CTAs per root repeat its set-up and, in CFR passes, pass every card's bucket
+// sums through memory. The estimate counts waves of one CTA per SM, in units of a river card's work
+// (8.2 us in single precision, about twice that in double): set-up 1, handing a card's sums over 0.4,
+// finish_kernel 5 (best responses, which have no bucket sums: 2). Measured on a pass pair (CFR of both
+// players), whole / split: 1 root 730 / 96 us, 20 roots 797 / 241, 74 roots 800 / 623; best responses in
+// double with host copies, 1 root 1207 / 143, 149 roots 3216 / 2362.
+int pick_splits(int n, int sms, bool cfr) {
+    if (n > kMaxSplitRoots) return 1;
+    int best = 1;
+    double least = (n + sms - 1) / sms * 49.0;
+    for (int s : {2, 3, 4, 6, 8, 12, 16, 24, 48}) {
+        const double cost = (double)((n * s + sms - 1) / sms) * (1.0 + 48 / s * (cfr ? 1.4 : 1.0)) + (cfr ? 5.0 : 2.0);
+        if (cost < 0.95 * least) {
+            least = cost;
+            best = s;
+        }
+    }
+    return best;
+}
+
+int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        return 148;
+    return sms;
+}
+
+size_t aligned(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+
 template <int MODE, typename V, bool AVG, int UPD>
 cudaError_t launch_upd(const SubgameDesc *desc, int n, const V *ranges, V *results, float *regrets,
                        const BoardPack *packs, unsigned long long flop, int max_groups, int max_card_groups,
-                       const float *own, float *avg, size_t smem, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(river_kernel<MODE, V, AVG, UPD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                       const float *own, float *avg, RiverScratch *scratch, cudaStream_t stream) {
+    constexpr int ACC = kNumLeaves + (AVG ? 1 : 0);
+    const Layout L = make_layout(MODE == kModeCFR, sizeof(V), max_groups, max_card_groups, ACC);
+    if (L.total > 227u * 1024u) return cudaErrorInvalidConfiguration;
+    const int splits = scratch ? pick_splits(n, sm_count(), MODE == kModeCFR) : 1;
+    if (splits > 1) {
+        const size_t outs = aligned((size_t)n * splits * kRangeStride * sizeof(V));
+        const size_t parts = MODE == kModeCFR ? (size_t)n * 48 * sizeof(RiverPart<ACC>) : 0;
+        unsigned char *mem = static_cast<unsigned char *>(scratch->take(outs + parts, stream));
+        if (mem) {
+            auto kernel = river_kernel<MODE, V, AVG, UPD, true>;
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+            if (e == cudaSuccess) {
+                kernel<<<n * splits, NT, L.total, stream>>>(desc, ranges, results, regrets, packs, flop, UPD, max_groups,
+                                                            max_card_groups, own, avg, splits,
+                                                            reinterpret_cast<V *>(mem), mem + outs);
+                e = cudaGetLastError();
+                cudaLaunchConfig_t cfg{};
+                cfg.gridDim = dim3(n, kBuckets / kFinBuckets);
+                cfg.blockDim = dim3(MODE == kModeCFR ? kFinThreads : 96);
+                cfg.stream = stream;
+                cudaLaunchAttribute attr{};
+                attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                attr.val.programmaticStreamSerializationAllowed = 1;
+                cfg.attrs = &attr;
+                cfg.numAttrs = 1;
+                if (e == cudaSuccess)
+                    e = cudaLaunchKernelEx(&cfg, finish_kernel<MODE, V, AVG, UPD>, desc, reinterpret_cast<const V *>(mem),
+                                           splits, (const void *)(mem + outs), results, regrets, avg);
+            }
+            scratch->give_back(mem, stream);
+            return e;
+        }
+    }
+    auto kernel = river_kernel<MODE, V, AVG, UPD, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
     if (e != cudaSuccess) return e;
-    river_kernel<MODE, V, AVG, UPD><<<n, NT, smem, stream>>>(desc, ranges, results, regrets, packs, flop, UPD,
-                                                             max_groups, max_card_groups, own, avg);
+    kernel<<<n, NT, L.total, stream>>>(desc, ranges, results, regrets, packs, flop, UPD, max_groups, max_card_groups, own,
+                                       avg, 1, nullptr, nullptr);
     return cudaGetLastError();
 }
 
 template <int MODE, typename V, bool AVG>
 cudaError_t launch_one(const SubgameDesc *desc, int n, const V *ranges, V *results, float *regrets,
                        const BoardPack *packs, unsigned long long flop, int updater, int max_groups,
-                       int max_card_groups, const float *own, float *avg, cudaStream_t stream) {
-    const Layout L = make_layout(MODE == kModeCFR, sizeof(V), max_groups, max_card_groups,
-                                 kNumLeaves + (AVG ? 1 : 0));
-    if (L.total > 227u * 1024u) return cudaErrorInvalidConfiguration;
+                       int max_card_groups, const float *own, float *avg, RiverScratch *scratch, cudaStream_t stream) {
     if (updater == 0)
         return launch_upd<MODE, V, AVG, 0>(desc, n, ranges, results, regrets, packs, flop, max_groups,
-                                           max_card_groups, own, avg, L.total, stream);
+                                           max_card_groups, own, avg, scratch, stream);
     return launch_upd<MODE, V, AVG, 1>(desc, n, ranges, results, regrets, packs, flop, max_groups, max_card_groups,
-                                       own, avg, L.total, stream);
+                                       own, avg, scratch, stream);
 }
 
 }  // namespace
+
+void *RiverScratch::take(size_t bytes, cudaStream_t stream) {
+    // an allocation inside a capture would become part of the caller's graph
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+                pool = nullptr;
+                cudaGetLastError();
+                return nullptr;
+            }
+            unsigned long long keep = kMaxScratch;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+    }
+    void *p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes, pool, stream) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+void RiverScratch::give_back(void *p, cudaStream_t stream) { cudaFreeAsync(p, stream); }
+
+RiverScratch::~RiverScratch() {
+    if (pool) cudaMemPoolDestroy(pool);
+}
 
 size_t river_smem_bytes(int mode, int fp64, int max_groups, int max_card_groups) {
     return make_layout(mode == kModeCFR, fp64 ? 8 : 4, max_groups, max_card_groups,
@@ -862,22 +1107,22 @@ size_t river_smem_bytes(int mode, int fp64, int max_groups, int max_card_groups)
 cudaError_t launch_river(int mode, const SubgameDesc *desc, int n, const float *ranges, float *results,
                          float *regrets, const BoardPack *packs, unsigned long long flop, int updater,
                          int max_groups, int max_card_groups, const float *own_ranges, float *avg_sums,
-                         cudaStream_t stream) {
+                         RiverScratch *scratch, cudaStream_t stream) {
     if (mode == kModeCFR && own_ranges && avg_sums)
         return launch_one<kModeCFR, float, true>(desc, n, ranges, results, regrets, packs, flop, updater,
-                                                 max_groups, max_card_groups, own_ranges, avg_sums, stream);
+                                                 max_groups, max_card_groups, own_ranges, avg_sums, scratch, stream);
     if (mode == kModeCFR)
         return launch_one<kModeCFR, float, false>(desc, n, ranges, results, regrets, packs, flop, updater,
-                                                  max_groups, max_card_groups, nullptr, nullptr, stream);
+                                                  max_groups, max_card_groups, nullptr, nullptr, scratch, stream);
     return launch_one<kModeBR, float, false>(desc, n, ranges, results, regrets, packs, flop, updater,
-                                             max_groups, max_card_groups, nullptr, nullptr, stream);
+                                             max_groups, max_card_groups, nullptr, nullptr, scratch, stream);
 }
 
 cudaError_t launch_river_br64(const SubgameDesc *desc, int n, const double *ranges, double *results,
                               float *regrets, const BoardPack *packs, unsigned long long flop, int updater,
-                              int max_groups, int max_card_groups, cudaStream_t stream) {
+                              int max_groups, int max_card_groups, RiverScratch *scratch, cudaStream_t stream) {
     return launch_one<kModeBR, double, false>(desc, n, ranges, results, regrets, packs, flop, updater,
-                                              max_groups, max_card_groups, nullptr, nullptr, stream);
+                                              max_groups, max_card_groups, nullptr, nullptr, scratch, stream);
 }
 
 }  // namespace prb
