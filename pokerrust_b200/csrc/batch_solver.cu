@@ -50,9 +50,9 @@ __global__ void __launch_bounds__(kSetupThreads) batch_setup_kernel(const BSub *
     BPack *pk = packs + s;
     __shared__ unsigned long long key[2048];
     __shared__ uint16_t hand_at[kBRow];
-    __shared__ uint16_t first[kBRow], last[kBRow];
-    __shared__ uint8_t lo_li[kBRow], hi_li[kBRow], lo_gs[kBRow], lo_ge[kBRow], hi_gs[kBRow], hi_ge[kBRow];
-    __shared__ uint8_t list_card[48];
+    __shared__ uint8_t lo_li[kBRow], hi_li[kBRow], lo_gi[kBRow], hi_gi[kBRow];  // list; group within it
+    __shared__ uint16_t gid[kBRow], lrow[48];
+    __shared__ uint8_t list_card[48], list_groups[48];
 
     if (__popcll(board) != 5 || (board >> 52)) {
         if (tid == 0) atomicOr(err, 1);
@@ -92,17 +92,17 @@ __global__ void __launch_bounds__(kSetupThreads) batch_setup_kernel(const BSub *
             if (!((board >> c) & 1)) list_card[n++] = (uint8_t)c;
         list_card[47] = 0;
         // tie groups: equal hand values
-        int f = 0;
+        int g = -1;
         for (int p = 0; p < kBLive; p++) {
-            if (p > 0 && (key[p] >> 11) != (key[p - 1] >> 11)) f = p;
-            first[p] = (uint16_t)f;
+            if (p == 0 || (key[p] >> 11) != (key[p - 1] >> 11)) {
+                if (g >= 0 && g < kBMaxGroups) pk->last[g] = (uint16_t)(p - 1);
+                g++;
+            }
+            gid[p] = (uint16_t)g;
         }
-        int l = kBLive - 1;
-        for (int p = kBLive - 1; p >= 0; p--) {
-            if (p < kBLive - 1 && (key[p] >> 11) != (key[p + 1] >> 11)) l = p;
-            last[p] = (uint16_t)l;
-        }
-        for (int p = kBLive; p < kBRow; p++) first[p] = last[p] = (uint16_t)p;
+        if (g >= kBMaxGroups) atomicOr(err, 4);
+        else pk->last[g] = (uint16_t)(kBLive - 1);
+        pk->num_groups = (uint16_t)(g + 1);
     }
     __syncthreads();
     if (tid < kBLists) {
@@ -119,38 +119,42 @@ __global__ void __launch_bounds__(kSetupThreads) batch_setup_kernel(const BSub *
         }
         if (k != kBListLen) atomicOr(err, 2);
         for (int j = 0; j < 48; j++) pk->clpos[li][j] = j < k ? pos[j] : (uint16_t)(kBRow - 1);
-        int j = 0;
-        while (j < k) {
-            int e = j;
-            while (e + 1 < k && first[pos[e + 1]] == first[pos[j]]) e++;
-            for (int q = j; q <= e; q++) {
-                int c1, c2;
-                hand_cards(hand_at[pos[q]], &c1, &c2);
-                if (c1 == card) {
-                    lo_li[pos[q]] = (uint8_t)li;
-                    lo_gs[pos[q]] = (uint8_t)j;
-                    lo_ge[pos[q]] = (uint8_t)e;
-                } else {
-                    hi_li[pos[q]] = (uint8_t)li;
-                    hi_gs[pos[q]] = (uint8_t)j;
-                    hi_ge[pos[q]] = (uint8_t)e;
-                }
+        int n = 0;
+        unsigned long long ends = 0;
+        for (int j = 0; j < k; j++) {
+            if (j == 0 || gid[pos[j]] != gid[pos[j - 1]]) n++;
+            if (j + 1 == k || gid[pos[j]] != gid[pos[j + 1]]) ends |= 1ull << j;
+            int c1, c2;
+            hand_cards(hand_at[pos[j]], &c1, &c2);
+            if (c1 == card) {
+                lo_li[pos[j]] = (uint8_t)li;
+                lo_gi[pos[j]] = (uint8_t)(n - 1);
+            } else {
+                hi_li[pos[j]] = (uint8_t)li;
+                hi_gi[pos[j]] = (uint8_t)(n - 1);
             }
-            j = e + 1;
         }
+        list_groups[li] = (uint8_t)n;
+        pk->ends[li] = make_uint2((uint32_t)ends, (uint32_t)(ends >> 32));
     }
-    if (tid == kBLists) {
-        for (int c = 0; c < 48; c++) pk->list_card[c] = list_card[c];
+    __syncthreads();
+    if (tid == 0) {
+        int r = 0;
+        for (int li = 0; li < kBLists; li++) {
+            lrow[li] = (uint16_t)r;
+            r += list_groups[li];
+        }
+        lrow[kBLists] = (uint16_t)r;
+        if (r > kBMaxRows) atomicOr(err, 8);
+        for (int li = 0; li < 48; li++) pk->lrow[li] = lrow[li];
     }
     __syncthreads();
     for (int p = tid; p < kBRow; p += kSetupThreads) {
         const bool live = p < kBLive;
-        pk->grp[p] = (uint32_t)first[p] | ((uint32_t)last[p] << 16);
-        pk->lists[p] = live ? ((uint32_t)lo_li[p] | ((uint32_t)hi_li[p] << 8) | ((uint32_t)lo_gs[p] << 16) |
-                               ((uint32_t)lo_ge[p] << 24))
-                            : 0u;
-        pk->lists2[p] = live ? ((uint32_t)hi_gs[p] | ((uint32_t)hi_ge[p] << 8)) : 0u;
+        pk->rows[p] = live ? (uint32_t)(lrow[lo_li[p]] + lo_gi[p]) | ((uint32_t)(lrow[hi_li[p]] + hi_gi[p]) << 16) : 0u;
+        pk->grp[p] = live ? (uint32_t)gid[p] | ((uint32_t)lo_li[p] << 16) | ((uint32_t)hi_li[p] << 24) : 0u;
         pk->hand[p] = hand_at[p];
+        pk->pgrp[p] = live ? (uint16_t)(gid[p] | (p + 1 == kBLive || gid[p + 1] != gid[p] ? 0x8000 : 0)) : 0;
     }
     for (int h = tid; h < 1328; h += kSetupThreads) pk->pos_of[h] = 0xFFFF;
     __syncthreads();
@@ -205,49 +209,86 @@ __device__ __forceinline__ void prefetch_subgame(const BLaunch &a, int s) {
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 
-template <typename V>
-struct Smem {
-    V *X;     // [group][kBRow] opponent weights, then leaf values
-    V *I;     // [2][kBRow] chunk-local inclusive scans
-    V *CT;    // [2][kBChunks] chunk totals
-    V *SC;    // [2][kBLists][48] inclusive scans of the card lists
-    BNode *tn;
-    uint16_t *leaf_node;
-    uint32_t *clpos;  // [kBLists][24] the card lists' positions, two per word (the pack's clpos)
-    V *wsum;  // [32] warp partial sums
+// Words of the pack that every leaf scan reads, staged once per subgame.
+struct PackWords {
+    uint32_t clpos[kBLists][24];  // the card lists' positions, two per word
+    uint2 ends[kBLists + 1];
+    uint16_t lrow[48];
+    uint16_t pgrp[kBRow];
+    uint16_t last[kBMaxGroups + 4];
+    uint16_t num_groups, pad[3];
 };
+static_assert(sizeof(PackWords) == offsetof(BPack, pos_of) - offsetof(BPack, clpos) && sizeof(PackWords) % 8 == 0,
+              "a piece of BPack");
+
+// A leaf, or a fold by the pass's player followed by its sibling call (see leaf_values).
+template <typename V>
+struct Job {
+    int x0;         // the scanned leaf's row in X, in values
+    int show;       // it is a showdown
+    V stake, fold;  // signed stakes of the scanned leaf and of the fold before it (0: none)
+};
+constexpr int kMaxGroupLeaves = 32;  // leaves of a group: a warp lays out its jobs
 
 template <typename V>
-__host__ __device__ inline size_t smem_bytes(int group) {
+struct Smem {
+    V *X;    // [group][kBRow] opponent weights, then leaf values
+    V *CT;   // [jobs][kCtRow] chunk totals of the rank order
+    V *PE;   // [jobs][kBMaxGroups] chunk-local prefix at each tie group's end
+    V *VG;   // [jobs][kBMaxGroups] W - B of each tie group
+    V *VC;   // [jobs][kVcRow] W - B of each row (tie group of a card list)
+    V *TL;   // [jobs][48] totals of the card lists
+    V *T;    // [jobs] totals
+    Job<V> *job;
+    BNode *tn;
+    uint16_t *leaf_node;
+    PackWords *words;
+    V *wsum;  // [32] warp partial sums
+};
+constexpr int kCtRow = 18, kVgRow = kBMaxGroups, kVcRow = 920, kTlRow = 48;
+static_assert(kBMaxRows <= kVcRow && kBChunks64 <= kCtRow, "rows");
+
+// Jobs whose scans run together: a thread takes a (job, card list) pair, so that 4 jobs give 188 tasks to
+// the 288 and 384 threads of K = 4 and 3 and 8 jobs 376 tasks to the 544 of K = 2.
+__host__ __device__ constexpr int jobs_of(int K, size_t value) { return K == 2 && value == 4 ? 8 : 4; }
+
+template <typename V>
+__host__ __device__ inline size_t smem_bytes(int group, int jobs) {
     size_t b = 0;
     b += (size_t)group * kBRow * sizeof(V);
-    b += 2 * (size_t)kBRow * sizeof(V);
-    b += 2 * (size_t)kBChunks * sizeof(V);
-    b += 2 * (size_t)kBLists * 48 * sizeof(V);
+    b += (size_t)jobs * (kCtRow + 2 * kVgRow + kVcRow + kTlRow + 2) * sizeof(V);
+    b += 32 * sizeof(V);
+    b += (size_t)kMaxGroupLeaves * sizeof(Job<V>);
     b += (size_t)kBMaxNodes * sizeof(BNode);
     b += (size_t)kBMaxLeaves * sizeof(uint16_t);
-    b += (size_t)kBLists * 48 * sizeof(uint16_t);
-    b += 32 * sizeof(V);
+    b += sizeof(PackWords);
     return (b + 15) & ~(size_t)15;
 }
 
 template <typename V>
-__device__ inline Smem<V> carve(unsigned char *base, int group) {
+__device__ inline Smem<V> carve(unsigned char *base, int group, int jobs) {
     Smem<V> S;
     V *v = reinterpret_cast<V *>(base);
     S.X = v;
     v += (size_t)group * kBRow;
-    S.I = v;
-    v += 2 * kBRow;
     S.CT = v;
-    v += 2 * kBChunks;
-    S.SC = v;
-    v += 2 * kBLists * 48;
+    v += jobs * kCtRow;
+    S.PE = v;
+    v += jobs * kVgRow;
+    S.VG = v;
+    v += jobs * kVgRow;
+    S.VC = v;
+    v += jobs * kVcRow;
+    S.TL = v;
+    v += jobs * kTlRow;
+    S.T = v;
+    v += jobs * 2;
     S.wsum = v;
     v += 32;
-    S.tn = reinterpret_cast<BNode *>(v);
+    S.job = reinterpret_cast<Job<V> *>(v);
+    S.tn = reinterpret_cast<BNode *>(S.job + kMaxGroupLeaves);
     S.leaf_node = reinterpret_cast<uint16_t *>(S.tn + kBMaxNodes);
-    S.clpos = reinterpret_cast<uint32_t *>(S.leaf_node + kBMaxLeaves);
+    S.words = reinterpret_cast<PackWords *>(S.leaf_node + kBMaxLeaves);
     return S;
 }
 
@@ -327,6 +368,172 @@ __device__ __forceinline__ V sigma(V val, V scale) {
     return scale < V(0) ? -scale : mul(val > V(0) ? val : V(0), scale);
 }
 
+// Lays out the jobs of the leaves [g0, g1) and returns their number; all warps call it, the first writes. A job is a leaf, or a fold
+// by p followed by its sibling call (a showdown): p's actions leave the opponent weights unchanged, so one
+// scan serves both leaves.
+template <typename V>
+__device__ __forceinline__ int lay_out_jobs(const Smem<V> &S, int g0, int g1, int p) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, j = g0 + lane;
+    BNode ln{};
+    if (j < g1) ln = S.tn[S.leaf_node[j]];
+    const int next_kind = __shfl_down_sync(FULL, (int)ln.kind, 1), next_parent = __shfl_down_sync(FULL, (int)ln.parent, 1);
+    const float next_stake = __shfl_down_sync(FULL, ln.stake, 1);
+    const bool pair = j + 1 < g1 && lane < 31 && ln.kind == kBFold && ln.actor == p && next_kind == kBShowdown &&
+                      next_parent == (int)ln.parent;
+    const unsigned pairs = __ballot_sync(FULL, pair), seconds = pairs << 1;
+    const bool start = j < g1 && !(seconds >> lane & 1);
+    const unsigned starts = __ballot_sync(FULL, start);
+    if (start && threadIdx.x < 32) {
+        Job<V> &job = S.job[__popc(starts & ((1u << lane) - 1))];
+        job.x0 = (lane + (pair ? 1 : 0)) * kBRow;
+        job.show = pair || ln.kind == kBShowdown;
+        job.stake = pair ? V(next_stake) : ln.kind == kBFold && ln.actor == p ? -V(ln.stake) : V(ln.stake);
+        job.fold = pair ? -V(ln.stake) : V(0);
+    }
+    return __popc(starts);
+}
+
+// The values of a group's leaves: opponent weights in X -> p's values, in place, for the jobs of
+// lay_out_jobs (n of them); all warps of the CTA call it. JOBS jobs go together:
+//   A  card lists, one thread per (job, list): the inclusive scan over the list's 23 pairs of hands in
+//      registers, by doubling steps, then W - B of every tie group of the list;
+//      rank order, on the warps left over: scans of 64-hand chunks, two hands per lane, of which the
+//      prefixes at the tie groups' ends are kept;
+//   B  W - B of every tie group of the rank order;
+//   C  values: a hand looks up its group and its two rows.
+// What bounds the phase is its instructions. A list scanned by a warp (23 of 32 lanes, five shuffles per
+// step) took about 110 of them per job, by a thread it takes 600 / 32. W - B formed per tie group (76 and
+// 542 on the mean board, for 1081 hands and 2162 list entries) has the operands it had per hand. Both
+// leave every bit as it was.
+template <int K, typename V, int NW, int JOBS>
+__device__ __forceinline__ void leaf_values(const Smem<V> &S, const BPack *__restrict__ pk, int n, int pos0) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kPairs = kBListLen / 2;
+    uint32_t rows[K], grp[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const int pq = pos0 + k < kBRow ? pos0 + k : kBRow - 1;
+        rows[k] = __ldg(&pk->rows[pq]);
+        grp[k] = __ldg(&pk->grp[pq]);
+    }
+    const PackWords &W = *S.words;
+#pragma unroll 1
+    for (int j0 = 0; j0 < n; j0 += JOBS) {
+        const int nj = min(JOBS, n - j0);
+        const int list_warps = (nj * kBLists + 31) / 32;  // fewer than NW
+        // ---- A ----
+        if (warp < list_warps) {
+            const int q = (int)threadIdx.x / kBLists, li = (int)threadIdx.x % kBLists;
+            if (q < nj) {
+                const V *x = S.X + S.job[j0 + q].x0;
+                V a0[kPairs], v[kPairs];
+#pragma unroll
+                for (int i = 0; i < kPairs; i++) {
+                    const uint32_t w = W.clpos[li][i];
+                    a0[i] = x[w & 0xFFFF];
+                    v[i] = a0[i] + x[w >> 16];
+                }
+#pragma unroll
+                for (int off = 1; off < kPairs; off <<= 1) {
+#pragma unroll
+                    for (int i = kPairs - 1; i >= off; i--) v[i] += v[i - off];
+                }
+                const V total = v[kPairs - 1];
+                const uint2 ends = W.ends[li];
+                V *to = S.VC + q * kVcRow + W.lrow[li];
+                V before = V(0);  // prefix at the end of the group before
+#pragma unroll
+                for (int i = 0; i < kPairs; i++) {
+                    const V even = (i > 0 ? v[i > 0 ? i - 1 : 0] : V(0)) + a0[i];
+                    if ((2 * i < 32 ? ends.x >> (2 * i) : ends.y >> (2 * i - 32)) & 1) {
+                        *to++ = (even + before) - total;
+                        before = even;
+                    }
+                    if ((2 * i + 1 < 32 ? ends.x >> (2 * i + 1) : ends.y >> (2 * i + 1 - 32)) & 1) {
+                        *to++ = (v[i] + before) - total;
+                        before = v[i];
+                    }
+                }
+                S.TL[q * kTlRow + li] = total;
+            }
+        } else {
+            for (int u = warp - list_warps; u < kBChunks64 * nj; u += NW - list_warps) {
+                const int q = u / kBChunks64, c = u - q * kBChunks64;
+                const V *x = S.X + S.job[j0 + q].x0 + c * 64 + 2 * lane;
+                const V a0 = x[0];
+                V v = a0 + x[1];
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const V t = __shfl_up_sync(FULL, v, off);
+                    if (lane >= off) v += t;
+                }
+                V ex = __shfl_up_sync(FULL, v, 1);
+                if (lane == 0) ex = V(0);
+                const uint32_t g = *reinterpret_cast<const uint32_t *>(W.pgrp + c * 64 + 2 * lane);
+                if (g & 0x8000u) S.PE[q * kVgRow + (g & 0x7FFF)] = ex + a0;
+                if (g & 0x80000000u) S.PE[q * kVgRow + (g >> 16 & 0x7FFF)] = v;
+                if (lane == 31) S.CT[q * kCtRow + c] = v;
+            }
+        }
+        __syncthreads();
+        // ---- B: a warp per job ----
+        for (int q = warp; q < nj; q += NW) {
+            V cofs = lane < kBChunks64 ? S.CT[q * kCtRow + lane] : V(0);  // chunk offsets: lane c holds chunk c's
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const V t = __shfl_up_sync(FULL, cofs, off);
+                if (lane >= off) cofs += t;
+            }
+            const V T = __shfl_sync(FULL, cofs, kBChunks64 - 1);
+            cofs = __shfl_up_sync(FULL, cofs, 1);
+            if (lane == 0) {
+                cofs = V(0);
+                S.T[q] = T;
+            }
+            const int G = W.num_groups;
+            for (int g0 = 0; g0 < G; g0 += 32) {
+                const int g = min(g0 + lane, G - 1);
+                const int ge = W.last[g], gs = g > 0 ? W.last[g > 0 ? g - 1 : 0] : 0;  // ends of this group and the one before
+                const V oe = __shfl_sync(FULL, cofs, ge >> 6), os = __shfl_sync(FULL, cofs, gs >> 6);
+                const V Pe = oe + S.PE[q * kVgRow + g];
+                const V Ps = g > 0 ? os + S.PE[q * kVgRow + (g > 0 ? g - 1 : 0)] : V(0);
+                if (g0 + lane < G) S.VG[q * kVgRow + g] = (Pe + Ps) - T;
+            }
+        }
+        __syncthreads();
+        // ---- C ----
+#pragma unroll 2
+        for (int q = 0; q < nj; q++) {
+            const Job<V> job = S.job[j0 + q];
+            V *x = S.X + job.x0;
+            V val[K];
+            if (job.show) {
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const V vg = S.VG[q * kVgRow + (grp[k] & 0xFFFF)];
+                    const V v1 = S.VC[q * kVcRow + (rows[k] & 0xFFFF)], v2 = S.VC[q * kVcRow + (rows[k] >> 16)];
+                    val[k] = pos0 + k < kBLive ? mul(job.stake, (vg - v1) - v2) : V(0);
+                }
+            }
+            if (!job.show || job.fold != V(0)) {
+                V xv[K], fold[K];
+                ld_k<K>(x, pos0, xv);
+                const V T = S.T[q], m = job.show ? job.fold : job.stake;
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const V t1 = S.TL[q * kTlRow + (grp[k] >> 16 & 255)], t2 = S.TL[q * kTlRow + (grp[k] >> 24)];
+                    fold[k] = pos0 + k < kBLive ? mul(m, ((T - t1) - t2) + xv[k]) : V(0);
+                }
+                st_k<K>(x - (job.show ? kBRow : 0), pos0, fold);
+            }
+            if (job.show) st_k<K>(x, pos0, val);
+        }
+        __syncthreads();  // the next jobs rewrite the scans
+    }
+}
+
 // MINB: CTAs per SM the registers are capped for (Cfg<K>::MINB, or 3 for the dense K = 4
 // configuration with 10-leaf groups).
 template <int K, typename V, int MODE, bool AVG, bool USEAVG, int MINB>
@@ -336,7 +543,8 @@ __global__ void __launch_bounds__(Cfg<K>::NT, MINB) batch_kernel(BLaunch a, int 
     static_assert(MODE == kBModeCFR || !AVG, "average sums accumulate in CFR passes");
     static_assert(MODE != kBModeCFR || (sizeof(V) == 4 && !USEAVG), "CFR runs on regrets in single precision");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem<V> S = carve<V>(smem_raw, group);
+    constexpr int kJobs = jobs_of(K, sizeof(V));
+    Smem<V> S = carve<V>(smem_raw, group, kJobs);
     __shared__ int s_next;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -371,10 +579,10 @@ __global__ void __launch_bounds__(Cfg<K>::NT, MINB) batch_kernel(BLaunch a, int 
             S.tn[i] = nd;
             if (nd.kind != kBDecision) S.leaf_node[nd.edge] = (uint16_t)i;
         }
-        // the card lists' positions, read by every leaf scan, staged once per subgame
         {
-            const uint32_t *src = reinterpret_cast<const uint32_t *>(&pk->clpos[0][0]);
-            for (int i = tid; i < kBLists * 24; i += NT) S.clpos[i] = __ldg(src + i);
+            const uint2 *src = reinterpret_cast<const uint2 *>(&pk->clpos[0][0]);
+            uint2 *dst = reinterpret_cast<uint2 *>(S.words);
+            for (int i = tid; i < (int)(sizeof(PackWords) / 8); i += NT) dst[i] = __ldg(src + i);
         }
         __syncthreads();
         float *R = a.regrets + (size_t)sub.edge_off * kBRow;
@@ -382,7 +590,6 @@ __global__ void __launch_bounds__(Cfg<K>::NT, MINB) batch_kernel(BLaunch a, int 
         const float *Src = src_all + (size_t)sub.edge_off * kBRow;
         const float *rng = a.ranges + (size_t)s * 2 * kBRow;
         const int pos0 = tid * K;
-        // this thread's hands' tie-group and card-list bounds, read once per subgame
 
         // walker state, per owned hand: depth-indexed stacks of the open path (indexed at run
         // time, so they live in local memory, cached in L1). Depth-major with the K hands of a
@@ -564,195 +771,12 @@ __global__ void __launch_bounds__(Cfg<K>::NT, MINB) batch_kernel(BLaunch a, int 
                     st_k<K>(S.X + (size_t)(nd.edge - g0) * kBRow, pos0, xv);
                 }
             }
+            // (every warp counts them, the first writes them)
+            const int jobs = lay_out_jobs(S, g0, g1, p);
             __syncthreads();
 
             // ---- leaves of the group: opponent weights -> p's values ----
-            // this thread's hands' tie-group and card-list bounds (read here rather than kept
-            // in registers through the walks)
-            uint32_t pgrp[K], plist[K], plist2[K];
-    #pragma unroll
-            for (int k = 0; k < K; k++) {
-                const int pq = pos0 + k < kBRow ? pos0 + k : kBRow - 1;
-                pgrp[k] = __ldg(&pk->grp[pq]);
-                plist[k] = __ldg(&pk->lists[pq]);
-                plist2[k] = __ldg(&pk->lists2[pq]);
-            }
-            // A job is a leaf, or a fold by p followed by its sibling call (a showdown): p's
-            // actions leave the opponent weights unchanged, so one scan serves both leaves.
-            // Jobs go kJ at a time. With kJ = 2 (buffers 0 and 1) their scans interleave and
-            // each hand's tie-group and card-list bounds are unpacked once for both; the dense
-            // configuration (MINB = 3) runs one job at a time in alternate buffers instead,
-            // which needs no barrier after the values and fits its register cap. Every job's
-            // arithmetic is the same either way.
-            constexpr int kJ = MINB >= 3 ? 1 : 2;
-            int batch_no = 0;
-            for (int j = g0; j < g1; batch_no++) {
-                // buffer of job q of this step
-                auto bufq = [&](int q) { return kJ == 1 ? (batch_no & 1) : q; };
-                bool pair[2] = {false, false};
-                BNode ln[2], lsd[2];
-                V *xs[2], *xfs[2];
-                int nj = 0;
-                while (nj < kJ && j < g1) {
-                    ln[nj] = S.tn[S.leaf_node[j]];
-                    lsd[nj] = ln[nj];  // the leaf whose kind and stake give the main value
-                    if (ln[nj].kind == kBFold && ln[nj].actor == p && j + 1 < g1) {
-                        const BNode nx = S.tn[S.leaf_node[j + 1]];
-                        if (nx.kind == kBShowdown && nx.parent == ln[nj].parent) {
-                            pair[nj] = true;
-                            lsd[nj] = nx;
-                        }
-                    }
-                    xfs[nj] = S.X + (size_t)(j - g0) * kBRow;          // the fold's row when paired
-                    xs[nj] = pair[nj] ? xfs[nj] + kBRow : xfs[nj];     // the scanned leaf's row
-                    j += pair[nj] ? 2 : 1;
-                    nj++;
-                }
-                // phase A: scans of the rank order in 64-hand chunks (two hands per lane) and
-                // scans of the card lists, unit u of both jobs together
-                for (int u = warp; u < kBChunks64 + kBLists; u += NW) {
-                    if (u < kBChunks64) {
-                        V a0[2], v[2];
-#pragma unroll
-                        for (int q = 0; q < kJ; q++) {
-                            a0[q] = v[q] = V(0);
-                            if (q < nj) {
-                                a0[q] = xs[q][u * 64 + 2 * lane];
-                                v[q] = a0[q] + xs[q][u * 64 + 2 * lane + 1];
-                            }
-                        }
-#pragma unroll
-                        for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-                            for (int q = 0; q < kJ; q++) {
-                                const V t = __shfl_up_sync(FULL, v[q], off);
-                                if (lane >= off) v[q] += t;
-                            }
-                        }
-#pragma unroll
-                        for (int q = 0; q < kJ; q++) {
-                            V ex = __shfl_up_sync(FULL, v[q], 1);
-                            if (lane == 0) ex = V(0);
-                            if (q < nj) {
-                                V *I = S.I + bufq(q) * kBRow;
-                                I[u * 64 + 2 * lane] = ex + a0[q];
-                                I[u * 64 + 2 * lane + 1] = v[q];
-                                if (lane == 31) S.CT[bufq(q) * kBChunks + u] = v[q];
-                            }
-                        }
-                    } else {
-                        const int li = u - kBChunks64;
-                        int c0 = 0, c1 = 0;
-                        if (lane < kBListLen / 2) {
-                            const uint32_t w = S.clpos[li * 24 + lane];
-                            c0 = w & 0xFFFF;
-                            c1 = w >> 16;
-                        }
-                        V a0[2], v[2];
-#pragma unroll
-                        for (int q = 0; q < kJ; q++) {
-                            a0[q] = v[q] = V(0);
-                            if (q < nj && lane < kBListLen / 2) {
-                                a0[q] = xs[q][c0];
-                                v[q] = a0[q] + xs[q][c1];
-                            }
-                        }
-#pragma unroll
-                        for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-                            for (int q = 0; q < kJ; q++) {
-                                const V t = __shfl_up_sync(FULL, v[q], off);
-                                if (lane >= off) v[q] += t;
-                            }
-                        }
-#pragma unroll
-                        for (int q = 0; q < kJ; q++) {
-                            V ex = __shfl_up_sync(FULL, v[q], 1);
-                            if (lane == 0) ex = V(0);
-                            if (q < nj && lane < kBListLen / 2) {
-                                V *SC = S.SC + bufq(q) * kBLists * 48;
-                                SC[li * 48 + 2 * lane] = ex + a0[q];
-                                SC[li * 48 + 2 * lane + 1] = v[q];
-                            }
-                        }
-                    }
-                }
-                __syncthreads();
-                // phase C: chunk offsets (every warp, same arithmetic; lane c holds chunk c's),
-                // then values
-                V cofs[2], T[2];
-                {
-                    V inc[2];
-#pragma unroll
-                    for (int q = 0; q < kJ; q++) inc[q] = (q < nj && lane < kBChunks64) ? S.CT[bufq(q) * kBChunks + lane] : V(0);
-#pragma unroll
-                    for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-                        for (int q = 0; q < kJ; q++) {
-                            const V t = __shfl_up_sync(FULL, inc[q], off);
-                            if (lane >= off) inc[q] += t;
-                        }
-                    }
-#pragma unroll
-                    for (int q = 0; q < kJ; q++) {
-                        cofs[q] = __shfl_up_sync(FULL, inc[q], 1);
-                        if (lane == 0) cofs[q] = V(0);
-                        T[q] = __shfl_sync(FULL, inc[q], kBChunks64 - 1);
-                    }
-                }
-                V xv[2][K], fv[2][K];
-#pragma unroll
-                for (int q = 0; q < kJ; q++)
-                    if (q < nj) ld_k<K>(xs[q], pos0, xv[q]);
-#pragma unroll
-                for (int k = 0; k < K; k++) {
-                    const int pos = pos0 + k;
-                    const uint32_t gr = pgrp[k], l1 = plist[k], l2 = plist2[k];
-                    const int gs = gr & 0xFFFF, ge = gr >> 16;
-                    const int li1 = l1 & 255, li2 = (l1 >> 8) & 255;
-                    const int gs1 = (l1 >> 16) & 255, ge1 = l1 >> 24;
-                    const int gs2 = l2 & 255, ge2 = (l2 >> 8) & 255;
-                    const int ce = ge >> 6, cs = gs > 0 ? (gs - 1) >> 6 : 0;
-#pragma unroll
-                    for (int q = 0; q < kJ; q++) {
-                        if (q >= nj) continue;
-                        // chunk offsets by shuffle (all lanes take part)
-                        const V oe = __shfl_sync(FULL, cofs[q], ce);
-                        const V os = __shfl_sync(FULL, cofs[q], cs);
-                        const V *I = S.I + bufq(q) * kBRow;
-                        const V *SC = S.SC + bufq(q) * kBLists * 48;
-                        V val = V(0), fval = V(0);
-                        if (pos < kBLive) {
-                            const V *sc1 = SC + li1 * 48;
-                            const V *sc2 = SC + li2 * 48;
-                            const V T1 = sc1[kBListLen - 1], T2 = sc2[kBListLen - 1];
-                            const V free = ((T[q] - T1) - T2) + xv[q][k];
-                            const V stake = V(lsd[q].stake);
-                            if (lsd[q].kind == kBShowdown) {
-                                const V Pe = oe + I[ge];
-                                const V Ps = gs > 0 ? os + I[gs - 1] : V(0);
-                                const V vg = (Pe + Ps) - T[q];
-                                const V v1 = (sc1[ge1] + (gs1 > 0 ? sc1[gs1 - 1] : V(0))) - T1;
-                                const V v2 = (sc2[ge2] + (gs2 > 0 ? sc2[gs2 - 1] : V(0))) - T2;
-                                val = mul(stake, (vg - v1) - v2);
-                            } else {
-                                val = mul(lsd[q].actor == p ? -stake : stake, free);
-                            }
-                            if (pair[q]) fval = mul(-V(ln[q].stake), free);
-                        }
-                        xv[q][k] = val;
-                        fv[q][k] = fval;
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < kJ; q++) {
-                    if (q >= nj) continue;
-                    st_k<K>(xs[q], pos0, xv[q]);
-                    if (pair[q]) st_k<K>(xfs[q], pos0, fv[q]);
-                }
-                if constexpr (kJ == 2) __syncthreads();  // the next two jobs rewrite buffers 0 and 1
-            }
-            if constexpr (kJ == 1) __syncthreads();  // the bottom-up walk reads every leaf's values
+            leaf_values<K, V, NW, kJobs>(S, pk, jobs, pos0);
 
             // ---- bottom-up walk over nodes [bu, end) ----
             unpark();
@@ -832,7 +856,7 @@ __global__ void weight_step_kernel(float *w) { *w += 1.0f; }
 
 template <int K, typename V, int MODE, bool AVG, bool USEAVG, int MINB = Cfg<K>::MINB>
 cudaError_t launch_one(const BLaunch &a, int ctas, int group, cudaStream_t stream) {
-    const size_t smem = smem_bytes<V>(group);
+    const size_t smem = smem_bytes<V>(group, jobs_of(K, sizeof(V)));
     cudaError_t e = cudaFuncSetAttribute(batch_kernel<K, V, MODE, AVG, USEAVG, MINB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -883,8 +907,7 @@ int batch_group_leaves(int fp64) { return fp64 ? 8 : 16; }
 int batch_dense_group() { return 9; }
 
 size_t batch_smem_bytes(int K, int fp64, int group) {
-    (void)K;
-    return fp64 ? smem_bytes<double>(group) : smem_bytes<float>(group);
+    return fp64 ? smem_bytes<double>(group, jobs_of(K, 8)) : smem_bytes<float>(group, jobs_of(K, 4));
 }
 
 cudaError_t launch_weight_step(float *w, cudaStream_t stream) {
@@ -894,7 +917,7 @@ cudaError_t launch_weight_step(float *w, cudaStream_t stream) {
 
 cudaError_t launch_batch_pass(int mode, int K, int fp64, int avg, const BLaunch &a, int ctas, int group,
                               cudaStream_t stream, int dense) {
-    if (group < 1 || group > kBMaxLeaves || ctas < 1) return cudaErrorInvalidValue;
+    if (group < 1 || group > kMaxGroupLeaves || ctas < 1) return cudaErrorInvalidValue;
     switch (K) {
         case 2: return launch_k<2>(mode, fp64, avg, a, ctas, group, stream, 0);
         case 3: return launch_k<3>(mode, fp64, avg, a, ctas, group, stream, 0);
@@ -905,7 +928,7 @@ cudaError_t launch_batch_pass(int mode, int K, int fp64, int avg, const BLaunch 
 
 int batch_dense_ctas_per_sm(int avg) {
     int n = 0;
-    const size_t smem = smem_bytes<float>(batch_dense_group());
+    const size_t smem = smem_bytes<float>(batch_dense_group(), jobs_of(4, 4));
     cudaError_t e;
     if (avg) {
         cudaFuncSetAttribute(batch_kernel<4, float, kBModeCFR, true, false, 3>,

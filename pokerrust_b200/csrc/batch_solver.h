@@ -14,7 +14,6 @@ constexpr int kBLive = 1081;   // hands that share no card with a 5-card board
 constexpr int kBRow = 1088;    // per-hand rows, padded to a multiple of 32
 constexpr int kBLists = 47;    // off-board cards
 constexpr int kBListLen = 46;  // live hands holding one off-board card
-constexpr int kBChunks = kBRow / 32;
 constexpr int kBChunks64 = kBRow / 64;  // 64-hand chunks of the rank-order scan
 
 // One subgame as the kernels see it.
@@ -26,20 +25,28 @@ struct BSub {
     float pot;
 };
 
+constexpr int kBMaxGroups = 136;  // tie groups of the live hands: the most any 5-card board has,
+constexpr int kBMaxRows = 917;    // and over its 47 card lists (both counted over all boards)
+
 // Per-subgame hand layout, built on the device from the board. Hands are held in rank
-// order ("positions"), weakest first, positions kBLive.. kBRow-1 are padding.
+// order ("positions"), weakest first, positions kBLive.. kBRow-1 are padding. The tie groups of each
+// card list are numbered through ("rows"), lists in card order.
 struct BPack {
-    uint32_t grp[kBRow];             // first | last position of the tie group << 16
-    uint32_t lists[kBRow];           // list of the low card | list of the high card << 8 |
-                                     //   first << 16 | last << 24 index of the tie group in the low card's list
-    uint32_t lists2[kBRow];          // first | last << 8: the same in the high card's list
+    uint32_t rows[kBRow];            // row of the hand's group in its low card's list | in its high card's << 16
+    uint32_t grp[kBRow];             // tie group | list of the low card << 16 | list of the high card << 24
     uint16_t hand[kBRow];            // colex hand index of each position (0xFFFF: padding)
     uint16_t clpos[kBLists][48];     // positions holding each off-board card, in rank order
-    uint8_t list_card[48];
+    uint2 ends[kBLists + 1];         // per list, bit j: its j-th hand is the last of its group
+    uint16_t lrow[48];               // first row of each list
+    uint16_t pgrp[kBRow];            // tie group of each position | 0x8000 at the group's last position
+    uint16_t last[kBMaxGroups + 4];  // last position of each tie group
+    uint16_t num_groups, pad[3];
     uint16_t pos_of[1328];           // position of each colex hand (0xFFFF: blocked)
 };
 
-static_assert(offsetof(BPack, clpos) % 4 == 0 && sizeof(BPack) % 4 == 0, "card lists move as 4-byte words");
+static_assert(offsetof(BPack, clpos) % 16 == 0 && sizeof(BPack) % 16 == 0 && sizeof(uint16_t[kBLists][48]) % 16 == 0 &&
+                  sizeof(uint16_t[48]) % 8 == 0 && sizeof(uint16_t[kBMaxGroups + 4]) % 8 == 0 && kBListLen <= 64,
+              "clpos to num_groups move as 8-byte words");
 
 enum { kBModeCFR = 0, kBModeBR = 1, kBModeEval = 2 };
 
