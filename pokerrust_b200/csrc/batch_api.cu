@@ -43,6 +43,7 @@ struct ClassCfg {
     int K = 2;                 // hands per thread
     int per_sm = 1;            // resident CTAs per SM
     int order = 0;             // 0: most work first, 1: input order
+    bool checks = false;       // every tree is check, check, showdown (no chips behind)
 };
 
 constexpr int kClasses = 2;    // trees with <= 16 leaves / more
@@ -140,6 +141,12 @@ struct Batch {
             a.ranges64 = fp64 ? d_ranges64 : nullptr;
             a.own_reach = own_weight;
             a.avg_weight = avg_weight;
+            if (k.checks && mode == kBModeCFR && !sum_out && !child_out) {
+                // such a class has its own kernel, whatever the configuration of the others
+                cudaError_t e = launch_check_pass(avg_on, a, sms, on ? on : stream);
+                if (e != cudaSuccess) return bfail("pass launch", e);
+                continue;
+            }
             const int ctas = std::min(k.count, std::max(1, k.per_sm) * sms);
             const int dense = mode == kBModeCFR && !fp64 && k.K == 4 && k.per_sm >= 3;
             const int group = dense ? batch_dense_group() : batch_group_leaves(fp64);
@@ -421,9 +428,12 @@ void *pr_batch_new(const pr_subgame *specs, int count, const float *ranges) {
     for (int c = 0; c < kClasses; c++) {
         b->cls[c].first = first;
         b->cls[c].count = 0;
+        b->cls[c].checks = true;
         for (int s = 0; s < count; s++)
             if ((b->subs[s].num_leaves > batch_group_leaves(0)) == (c == 1)) {
                 b->cls[c].count++;
+                // the only tree with one leaf is check, check, showdown
+                b->cls[c].checks &= b->subs[s].num_leaves == 1 && b->subs[s].num_edges == 2;
                 b->cls[c].max_leaves = std::max(b->cls[c].max_leaves, b->subs[s].num_leaves);
             }
         first += b->cls[c].count;
@@ -943,14 +953,18 @@ int pr_batch_tune(void *batch, double *ms_out) {
         float best = 1e30f;
         ClassCfg best_cfg = keep[c];
         for (int K : {2, 3, 4}) {
+            // a class of checks runs its own kernel under every configuration: keep the one it has
+            if (keep[c].checks && K != keep[c].K) continue;
             const int fits = batch_ctas_per_sm(kBModeCFR, K, 0, b->avg_on);
             // per = 1, 2 where they fit; K = 4 also tries the dense configuration (registers
             // capped for 3 CTAs per SM) where three of its CTAs fit
             std::vector<int> pers;
             for (int per = 1; per <= std::min(fits, 2); per++) pers.push_back(per);
             if (K == 4 && batch_dense_ctas_per_sm(b->avg_on) >= 3) pers.push_back(3);
+            if (keep[c].checks) pers.assign(1, keep[c].per_sm);
             for (int per : pers) {
                 for (int ord = 0; ord < 2; ord++) {
+                    if (keep[c].checks && ord != keep[c].order) continue;
                     for (int i = 0; i < kClasses; i++) b->cls[i] = keep[i];
                     b->cls[c].K = K;
                     b->cls[c].per_sm = per;

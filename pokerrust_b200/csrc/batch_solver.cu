@@ -394,6 +394,34 @@ __device__ __forceinline__ int lay_out_jobs(const Smem<V> &S, int g0, int g1, in
     return __popc(starts);
 }
 
+// A card list's rows, by one thread: a0 holds the first hand of each of its pairs, v the pairs' sums.
+// Writes W - B of every tie group of the list (bit j of `ends`: hand j is a group's last) and returns the
+// list's total.
+template <typename V>
+__device__ __forceinline__ V scan_list(const V (&a0)[kBListLen / 2], V (&v)[kBListLen / 2], uint2 ends, V *to) {
+    constexpr int kPairs = kBListLen / 2;
+#pragma unroll
+    for (int off = 1; off < kPairs; off <<= 1) {
+#pragma unroll
+        for (int i = kPairs - 1; i >= off; i--) v[i] += v[i - off];
+    }
+    const V total = v[kPairs - 1];
+    V before = V(0);  // prefix at the end of the group before
+#pragma unroll
+    for (int i = 0; i < kPairs; i++) {
+        const V even = (i > 0 ? v[i > 0 ? i - 1 : 0] : V(0)) + a0[i];
+        if ((2 * i < 32 ? ends.x >> (2 * i) : ends.y >> (2 * i - 32)) & 1) {
+            *to++ = (even + before) - total;
+            before = even;
+        }
+        if ((2 * i + 1 < 32 ? ends.x >> (2 * i + 1) : ends.y >> (2 * i + 1 - 32)) & 1) {
+            *to++ = (v[i] + before) - total;
+            before = v[i];
+        }
+    }
+    return total;
+}
+
 // The values of a group's leaves: opponent weights in X -> p's values, in place, for the jobs of
 // lay_out_jobs (n of them); all warps of the CTA call it. JOBS jobs go together:
 //   A  card lists, one thread per (job, list): the inclusive scan over the list's 23 pairs of hands in
@@ -435,27 +463,7 @@ __device__ __forceinline__ void leaf_values(const Smem<V> &S, const BPack *__res
                     a0[i] = x[w & 0xFFFF];
                     v[i] = a0[i] + x[w >> 16];
                 }
-#pragma unroll
-                for (int off = 1; off < kPairs; off <<= 1) {
-#pragma unroll
-                    for (int i = kPairs - 1; i >= off; i--) v[i] += v[i - off];
-                }
-                const V total = v[kPairs - 1];
-                const uint2 ends = W.ends[li];
-                V *to = S.VC + q * kVcRow + W.lrow[li];
-                V before = V(0);  // prefix at the end of the group before
-#pragma unroll
-                for (int i = 0; i < kPairs; i++) {
-                    const V even = (i > 0 ? v[i > 0 ? i - 1 : 0] : V(0)) + a0[i];
-                    if ((2 * i < 32 ? ends.x >> (2 * i) : ends.y >> (2 * i - 32)) & 1) {
-                        *to++ = (even + before) - total;
-                        before = even;
-                    }
-                    if ((2 * i + 1 < 32 ? ends.x >> (2 * i + 1) : ends.y >> (2 * i + 1 - 32)) & 1) {
-                        *to++ = (v[i] + before) - total;
-                        before = v[i];
-                    }
-                }
+                const V total = scan_list(a0, v, W.ends[li], S.VC + q * kVcRow + W.lrow[li]);
                 S.TL[q * kTlRow + li] = total;
             }
         } else {
@@ -737,7 +745,7 @@ __global__ void __launch_bounds__(Cfg<K>::NT, MINB) batch_kernel(BLaunch a, int 
                             float av[K];
                             ld_k<K>(A + ro, pos0, av);
 #pragma unroll
-                            for (int k = 0; k < K; k++) av[k] += wavg * float(npp[k]);
+                            for (int k = 0; k < K; k++) av[k] = __fmaf_rn(wavg, float(npp[k]), av[k]);
                             st_k<K>(A + ro, pos0, av);
                         }
                     }
@@ -852,6 +860,160 @@ __global__ void __launch_bounds__(Cfg<K>::NT, MINB) batch_kernel(BLaunch a, int 
     }
 }
 
+// Subgames without a bet (both players check, then the showdown: all-in river leaves) in CFR passes. Their
+// tree is two edges and one leaf, so that batch_kernel spends its time on the staging of tree and pack, the
+// walks' stacks and barriers, with at most three CTAs per SM: 1028 us for 18,816 of them. Here a CTA keeps
+// no tree, stack or leaf group: 9 KB of shared memory and 3 barriers per subgame, so that 4 share an SM
+// while the next subgame's rows are asked from L2. That takes 200 us (592: 32 -> 9 us), 4.2 TB/s of the 44 KB
+// that a subgame moves (pack, ranges, two regret rows, one sum row, root values); what is left is the wait
+// for those rows. 3 CTAs per SM took 215 us, 5 (40 registers, spills) 238.
+// The arithmetic is batch_kernel's, operand for operand. As there, a thread scans a card list: by a warp per
+// list the pass had 9,070 instructions per subgame and took 298 us, so it has 5,560.
+constexpr int kCheckCtas = 4;
+constexpr int kCheckThreads = 288;
+
+template <bool AVG>
+__global__ void __launch_bounds__(kCheckThreads, kCheckCtas) check_kernel(BLaunch a) {
+    constexpr int K = 4, NW = kCheckThreads / 32, kPairs = kBListLen / 2, kListWarps = (kBLists + 31) / 32;
+    __shared__ __align__(16) float X[kBRow];
+    __shared__ float CT[kCtRow], PE[kVgRow], VG[kVgRow], VC[kVcRow];
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, pos0 = tid * K;
+    const int p = a.player, o = 1 - p;
+    const float wavg = AVG && a.avg_weight ? *a.avg_weight : 1.0f;
+    int qi = blockIdx.x;
+    if (qi >= a.count) return;
+    int s = a.order[qi];
+    BSub sub = a.subs[s];
+    for (;;) {
+        const BPack *__restrict__ pk = a.packs + s;
+        float *R = a.regrets + (size_t)sub.edge_off * kBRow;  // rows: player 0's check, player 1's check
+        const float stake = a.nodes[sub.node_off + 2].stake;
+        // ---- opponent weights ----
+        float w[K], sv[K];
+        ld_k<K>(a.ranges + ((size_t)s * 2 + o) * kBRow, pos0, w);
+        ld_k<K>(R + (size_t)o * kBRow, pos0, sv);
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            w[k] = mul(w[k], sigma<float>(sv[k], strategy_scale<float, false>(sv[k] > 0.0f ? sv[k] : 0.0f, 1)));
+            if (pos0 + k >= kBLive) w[k] = 0.0f;
+        }
+        st_k<K>(X, pos0, w);
+        const int next = qi + gridDim.x;
+        int s_next = 0;
+        if (next < a.count) {
+            s_next = a.order[next];
+            sub = a.subs[s_next];
+            if (tid == 0) {
+                const BPack *nx = a.packs + s_next;
+                prefetch_l2(nx, offsetof(BPack, hand));
+                prefetch_l2(&nx->clpos[0][0], sizeof(PackWords) / 16 * 16);
+                prefetch_l2(a.ranges + (size_t)s_next * 2 * kBRow, 2 * kBRow * sizeof(float));
+                prefetch_l2(a.regrets + (size_t)sub.edge_off * kBRow, 2 * kBRow * sizeof(float));
+                if (AVG) prefetch_l2(a.avg + (size_t)(sub.edge_off + p) * kBRow, kBRow * sizeof(float));
+            }
+        }
+        __syncthreads();
+        // ---- scans: card lists on the first two warps, 64-hand chunks of the rank order on the others ----
+        if (warp < kListWarps) {
+            if (tid < kBLists) {
+                const uint4 *at = reinterpret_cast<const uint4 *>(&pk->clpos[tid][0]);
+                const uint2 ends = __ldg(&pk->ends[tid]);
+                float *to = VC + __ldg(&pk->lrow[tid]);
+                float a0[kPairs], v[kPairs];
+#pragma unroll
+                for (int j = 0; j < (kPairs + 3) / 4; j++) {
+                    const uint4 w4 = __ldg(at + j);
+                    const uint32_t w1[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        const int i = 4 * j + t;
+                        if (i >= kPairs) continue;
+                        a0[i] = X[w1[t] & 0xFFFF];
+                        v[i] = a0[i] + X[w1[t] >> 16];
+                    }
+                }
+                scan_list(a0, v, ends, to);
+            }
+        } else {
+            for (int c = warp - kListWarps; c < kBChunks64; c += NW - kListWarps) {
+                const float2 x2 = *reinterpret_cast<const float2 *>(X + c * 64 + 2 * lane);
+                float v = x2.x + x2.y;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const float t = __shfl_up_sync(FULL, v, off);
+                    if (lane >= off) v += t;
+                }
+                float ex = __shfl_up_sync(FULL, v, 1);
+                if (lane == 0) ex = 0.0f;
+                const uint32_t g = __ldg(reinterpret_cast<const uint32_t *>(pk->pgrp + c * 64) + lane);
+                if (g & 0x8000u) PE[g & 0x7FFF] = ex + x2.x;
+                if (g & 0x80000000u) PE[g >> 16 & 0x7FFF] = v;
+                if (lane == 31) CT[c] = v;
+            }
+        }
+        uint32_t rows[K], grp[K];
+        ld_k<K>(pk->rows, pos0, rows);
+        ld_k<K>(pk->grp, pos0, grp);
+        __syncthreads();
+        // ---- W - B of the tie groups of the rank order ----
+        const int G = __ldg(&pk->num_groups);
+        if (warp * 32 < G) {
+            float cofs = lane < kBChunks64 ? CT[lane] : 0.0f;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const float t = __shfl_up_sync(FULL, cofs, off);
+                if (lane >= off) cofs += t;
+            }
+            const float T = __shfl_sync(FULL, cofs, kBChunks64 - 1);
+            cofs = __shfl_up_sync(FULL, cofs, 1);
+            if (lane == 0) cofs = 0.0f;
+            const int g = min(tid, G - 1), gp = max(g - 1, 0);
+            const int ge = __ldg(&pk->last[g]), gs = g > 0 ? __ldg(&pk->last[gp]) : 0;
+            const float oe = __shfl_sync(FULL, cofs, ge >> 6), os = __shfl_sync(FULL, cofs, gs >> 6);
+            const float Pe = oe + PE[g], Ps = g > 0 ? os + PE[gp] : 0.0f;
+            if (tid < G) VG[g] = (Pe + Ps) - T;
+        }
+        // the own row, its sums and its reach while the groups are formed
+        float npp[K];
+        ld_k<K>(R + (size_t)p * kBRow, pos0, sv);
+        float scale[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) scale[k] = strategy_scale<float, false>(sv[k] > 0.0f ? sv[k] : 0.0f, 1);
+        if constexpr (AVG) {
+            if (a.own_reach) {
+                ld_k<K>(a.ranges + ((size_t)s * 2 + p) * kBRow, pos0, npp);
+            } else {
+#pragma unroll
+                for (int k = 0; k < K; k++) npp[k] = 1.0f;
+            }
+            float *A = a.avg + (R - a.regrets) + (size_t)p * kBRow;
+            float av[K];
+            ld_k<K>(A, pos0, av);
+#pragma unroll
+            for (int k = 0; k < K; k++) av[k] = __fmaf_rn(wavg, mul(npp[k], sigma<float>(sv[k], scale[k])), av[k]);
+            st_k<K>(A, pos0, av);
+        }
+        __syncthreads();
+        // ---- values; regrets of the own check; root ----
+        float r[K], root[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const float vg = VG[grp[k] & 0xFFFF], v1 = VC[rows[k] & 0xFFFF], v2 = VC[rows[k] >> 16];
+            float v = pos0 + k < kBLive ? mul(stake, (vg - v1) - v2) : 0.0f;
+            if (p == 0) v = 0.0f + v;  // passed through player 1's node
+            r[k] = sv[k] + v;
+            root[k] = 0.0f + mul(sigma<float>(sv[k], scale[k]), v);
+            r[k] = fmaxf(r[k] - root[k], 0.0f);
+        }
+        st_k<K>(R + (size_t)p * kBRow, pos0, r);
+        if (a.root_out) st_k<K>(reinterpret_cast<float *>(a.root_out) + (size_t)s * kBRow, pos0, root);
+        if (next >= a.count) break;
+        qi = next;
+        s = s_next;
+    }
+}
+
 __global__ void weight_step_kernel(float *w) { *w += 1.0f; }
 
 template <int K, typename V, int MODE, bool AVG, bool USEAVG, int MINB = Cfg<K>::MINB>
@@ -912,6 +1074,15 @@ size_t batch_smem_bytes(int K, int fp64, int group) {
 
 cudaError_t launch_weight_step(float *w, cudaStream_t stream) {
     weight_step_kernel<<<1, 1, 0, stream>>>(w);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_check_pass(int avg, const BLaunch &a, int sms, cudaStream_t stream) {
+    if (a.sum_out || a.child_out || (avg && !a.avg)) return cudaErrorInvalidValue;
+    if (a.count <= 0) return cudaSuccess;
+    const int most = kCheckCtas * sms, ctas = a.count < most ? a.count : most;
+    if (avg) check_kernel<true><<<ctas, kCheckThreads, 0, stream>>>(a);
+    else check_kernel<false><<<ctas, kCheckThreads, 0, stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -83,6 +83,10 @@ cudaError_t launch_batch_setup(const BSub *subs, int count, BPack *packs, const 
 cudaError_t launch_batch_pass(int mode, int K, int fp64, int avg, const BLaunch &a, int ctas, int max_leaves,
                               cudaStream_t stream, int dense = 0);
 
+// A CFR pass over a queue of subgames whose tree is check, check, showdown (nodes: player 0's decision,
+// player 1's, the showdown), without child or summed outputs. The queue head is not used.
+cudaError_t launch_check_pass(int avg, const BLaunch &a, int sms, cudaStream_t stream);
+
 // Adds 1 to the device scalar *w (the next iteration's average weight), on `stream`.
 cudaError_t launch_weight_step(float *w, cudaStream_t stream);
 
