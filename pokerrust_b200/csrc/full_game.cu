@@ -108,7 +108,14 @@ struct FView {
     const int *kids;
 };
 
-// ---- top-down: reach of both players ([node][2][kH]) ----
+// The sweeps' levels hold tens to a few thousand nodes of 1326 hands, and a launch lasts as long as its
+// slowest thread's chain of dependent loads. So a thread takes one hand of a node (kHandChunks CTAs per
+// node), and what every hand of a node reads goes through shared memory first. Of a flop game with 441
+// betting and 392 all-in turn leaves one iteration took 6.39 ms with a CTA per node, 5.75 ms so (with
+// value-network leaves 2.04 -> 1.46), the changes of scatter_kernel and gather_kernel included.
+constexpr int kHandChunks = (kH + FT - 1) / FT;
+
+// ---- top-down: reach of both players ([node][2][kH]); one CTA per (node, FT hands) ----
 template <typename T>
 __global__ void __launch_bounds__(FT) down_kernel(FView v, const int *__restrict__ level, T *__restrict__ R,
                                                    const float *__restrict__ src, int average) {
@@ -116,19 +123,17 @@ __global__ void __launch_bounds__(FT) down_kernel(FView v, const int *__restrict
     const FNode nd = v.nodes[n];
     const T *r0 = R + (size_t)n * 2 * kH;
     const T *r1 = r0 + kH;
-    if (nd.kind == kFDecision) {
-        for (int h = threadIdx.x; h < kH; h += FT) {
-            T p[kFMaxKids];
-            strategy<T>(src, nd.edge, nd.nchild, h, average != 0, p);
-            const T a = r0[h], b = r1[h];
+    const int h = blockIdx.y * FT + threadIdx.x;
+    if (nd.kind != kFDecision || h >= kH) return;
+    T p[kFMaxKids];
+    strategy<T>(src, nd.edge, nd.nchild, h, average != 0, p);
+    const T a = r0[h], b = r1[h];
 #pragma unroll
-            for (int k = 0; k < kFMaxKids; k++) {
-                if (k >= nd.nchild) break;
-                T *c = R + (size_t)v.kids[nd.kids + k] * 2 * kH;
-                c[h] = nd.actor == 0 ? mul(a, p[k]) : a;
-                c[kH + h] = nd.actor == 1 ? mul(b, p[k]) : b;
-            }
-        }
+    for (int k = 0; k < kFMaxKids; k++) {
+        if (k >= nd.nchild) break;
+        T *c = R + (size_t)v.kids[nd.kids + k] * 2 * kH;
+        c[h] = nd.actor == 0 ? mul(a, p[k]) : a;
+        c[kH + h] = nd.actor == 1 ? mul(b, p[k]) : b;
     }
 }
 
@@ -154,23 +159,30 @@ __global__ void __launch_bounds__(FT) deal_down_kernel(FView v, const int *__res
 // card count 0); one CTA per (deal node, FT hands)
 template <typename T>
 __global__ void __launch_bounds__(FT) deal_up_kernel(FView v, const int *__restrict__ deals, T *__restrict__ V) {
+    __shared__ int kid[52];
+    __shared__ unsigned long long dealt[52];
     const int n = deals[blockIdx.x];
     const FNode nd = v.nodes[n];
+    for (int k = threadIdx.x; k < nd.nchild; k += FT) {
+        kid[k] = v.kids[nd.kids + k];
+        dealt[k] = v.nodes[kid[k]].board & ~nd.board;
+    }
+    __syncthreads();
     const int h = blockIdx.y * FT + threadIdx.x;
     if (h >= kH) return;
     const unsigned long long hb = hand_bits(h);
     T s = T(0);
+#pragma unroll 8
     for (int k = 0; k < nd.nchild; k++) {
-        const int ci = v.kids[nd.kids + k];
-        if (hb & (v.nodes[ci].board & ~nd.board)) continue;
-        s += V[(size_t)ci * kH + h];
+        const T x = V[(size_t)kid[k] * kH + h];
+        if (!(hb & dealt[k])) s += x;
     }
     V[(size_t)n * kH + h] = s / T(nd.nchild);
 }
 
 enum { kUpCFR = 0, kUpBR = 1, kUpEval = 2 };
 
-// ---- bottom-up: values of `upd` ([node][kH]) ----
+// ---- bottom-up: values of `upd` ([node][kH]); one CTA per (node, FT hands), the first takes a fold ----
 template <typename T, int MODE>
 __global__ void __launch_bounds__(FT) up_kernel(FView v, const int *__restrict__ level, int upd,
                                                  const T *__restrict__ R, T *__restrict__ V,
@@ -179,22 +191,31 @@ __global__ void __launch_bounds__(FT) up_kernel(FView v, const int *__restrict__
                                                  int average, const float *__restrict__ wt) {
     __shared__ T red[FT];
     __shared__ T csum[52];
+    __shared__ T opp[kH];
     const int n = level[blockIdx.x];
     const FNode nd = v.nodes[n];
     T *out = V + (size_t)n * kH;
+    const int h = blockIdx.y * FT + threadIdx.x;
     switch (nd.kind) {
         case kFLeaf:
-            for (int h = threadIdx.x; h < kH; h += FT) out[h] = leafV[(size_t)nd.edge * kH + h];
+            if (h < kH) out[h] = leafV[(size_t)nd.edge * kH + h];
             return;
         case kFFold: {
-            // opponent weight compatible with each hand: total - both cards' sums + the hand
-            const T *opp = R + ((size_t)n * 2 + (1 - upd)) * kH;
+            // opponent weight compatible with each hand: total - both cards' sums + the hand. The cards'
+            // sums, 51 adds in a row each, read shared memory: from L2 they were half of a level's time.
+            if (blockIdx.y > 0) return;
+            const T *row = R + ((size_t)n * 2 + (1 - upd)) * kH;
             T part = T(0);
-            for (int h = threadIdx.x; h < kH; h += FT) part += opp[h];
+#pragma unroll
+            for (int i = 0; i < kHandChunks; i++) {
+                const int g = i * FT + threadIdx.x;
+                if (g < kH) part += opp[g] = row[g];
+            }
             const T total = cta_sum(part, red);
             if (threadIdx.x < 52) {
                 const int c = threadIdx.x;
                 T s = T(0);
+#pragma unroll 4
                 for (int o = 0; o < 52; o++) {
                     if (o == c) continue;
                     s += opp[c < o ? c + o * (o - 1) / 2 : o + c * (c - 1) / 2];
@@ -203,40 +224,39 @@ __global__ void __launch_bounds__(FT) up_kernel(FView v, const int *__restrict__
             }
             __syncthreads();
             const T m = T(nd.stake) * (nd.actor == upd ? T(-1) : T(1));
-            for (int h = threadIdx.x; h < kH; h += FT) {
+            for (int g = threadIdx.x; g < kH; g += FT) {
                 int c1, c2;
-                hand_cards(h, &c1, &c2);
-                const T x = ((total - csum[c1]) - csum[c2]) + opp[h];
-                out[h] = mul(m, x);
+                hand_cards(g, &c1, &c2);
+                const T x = ((total - csum[c1]) - csum[c2]) + opp[g];
+                out[g] = mul(m, x);
             }
             return;
         }
         default: {
+            if (h >= kH) return;
             const bool mine = nd.actor == upd;
             const T *own = R + ((size_t)n * 2 + upd) * kH;
             const float wavg = wt ? *wt : 1.0f;
-            for (int h = threadIdx.x; h < kH; h += FT) {
-                T p[kFMaxKids], u[kFMaxKids];
-                if (mine && MODE != kUpBR) strategy<T>(src, nd.edge, nd.nchild, h, average != 0, p);
-                T acc = (mine && MODE == kUpBR) ? neg_inf<T>() : T(0);
+            T p[kFMaxKids], u[kFMaxKids];
+            if (mine && MODE != kUpBR) strategy<T>(src, nd.edge, nd.nchild, h, average != 0, p);
+            T acc = (mine && MODE == kUpBR) ? neg_inf<T>() : T(0);
+#pragma unroll
+            for (int k = 0; k < kFMaxKids; k++) {
+                if (k >= nd.nchild) break;
+                u[k] = V[(size_t)v.kids[nd.kids + k] * kH + h];
+                if (!mine) acc += u[k];
+                else if (MODE == kUpBR) acc = acc > u[k] ? acc : u[k];
+                else acc += mul(p[k], u[k]);
+            }
+            out[h] = acc;
+            if (MODE == kUpCFR && mine) {
+                const T w = own[h];
 #pragma unroll
                 for (int k = 0; k < kFMaxKids; k++) {
                     if (k >= nd.nchild) break;
-                    u[k] = V[(size_t)v.kids[nd.kids + k] * kH + h];
-                    if (!mine) acc += u[k];
-                    else if (MODE == kUpBR) acc = acc > u[k] ? acc : u[k];
-                    else acc += mul(p[k], u[k]);
-                }
-                out[h] = acc;
-                if (MODE == kUpCFR && mine) {
-                    const T w = own[h];
-#pragma unroll
-                    for (int k = 0; k < kFMaxKids; k++) {
-                        if (k >= nd.nchild) break;
-                        float &r = regrets[(size_t)(nd.edge + k) * kH + h];
-                        r = fmaxf((r + float(u[k])) - float(acc), 0.0f);
-                        if (avg) avg[(size_t)(nd.edge + k) * kH + h] += wavg * float(mul(w, p[k]));
-                    }
+                    float &r = regrets[(size_t)(nd.edge + k) * kH + h];
+                    r = fmaxf((r + float(u[k])) - float(acc), 0.0f);
+                    if (avg) avg[(size_t)(nd.edge + k) * kH + h] += wavg * float(mul(w, p[k]));
                 }
             }
             return;
@@ -245,37 +265,65 @@ __global__ void __launch_bounds__(FT) up_kernel(FView v, const int *__restrict__
 }
 
 // ---- leaves <-> river subgames ----
-// subgame s belongs to slot s / 48 (a leaf node); its ranges are the leaf's reach.
+// subgame s belongs to slot s / 48 (a leaf node); its ranges are the leaf's reach. A CTA takes
+// kScatterRivers of a leaf's subgames: the reach goes to shared memory, where the gather by hand costs a
+// few bank conflicts instead of a cache line per lane.
+constexpr int kScatterRivers = 6;
 template <typename T>
 __global__ void __launch_bounds__(FT) scatter_kernel(const BPack *__restrict__ packs, const T *__restrict__ R,
                                                       const int *__restrict__ slot_node, T *__restrict__ ranges) {
-    const int s = blockIdx.x;
-    const T *r = R + (size_t)slot_node[s / kRivers] * 2 * kH;
-    const uint16_t *hand = packs[s].hand;
-    for (int p = threadIdx.x; p < kBRow; p += FT) {
-        const int h = hand[p];
-        ranges[((size_t)s * 2 + 0) * kBRow + p] = h != 0xFFFF ? r[h] : T(0);
-        ranges[((size_t)s * 2 + 1) * kBRow + p] = h != 0xFFFF ? r[kH + h] : T(0);
+    static_assert(kRivers % kScatterRivers == 0 && kBRow % 4 == 0 && offsetof(BPack, hand) % 8 == 0, "whole CTAs and quads");
+    __shared__ T r[2 * kH + 1];
+    const int s0 = blockIdx.x * kScatterRivers;
+    const T *row = R + (size_t)slot_node[s0 / kRivers] * 2 * kH;
+    for (int i = threadIdx.x; i < 2 * kH; i += FT) r[i] = row[i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < kScatterRivers * (kBRow / 4); i += FT) {
+        const int s = s0 + i / (kBRow / 4), q = i % (kBRow / 4);
+        const ushort4 h4 = *reinterpret_cast<const ushort4 *>(packs[s].hand + 4 * q);
+        const int h[4] = {h4.x, h4.y, h4.z, h4.w};
+#pragma unroll
+        for (int pl = 0; pl < 2; pl++) {
+            T x[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) x[t] = h[t] != 0xFFFF ? r[pl * kH + min(h[t], kH - 1)] : T(0);
+            T *to = ranges + ((size_t)s * 2 + pl) * kBRow + 4 * q;
+            if constexpr (sizeof(T) == 4) {
+                *reinterpret_cast<float4 *>(to) = make_float4(x[0], x[1], x[2], x[3]);
+            } else {
+                reinterpret_cast<double2 *>(to)[0] = make_double2(x[0], x[1]);
+                reinterpret_cast<double2 *>(to)[1] = make_double2(x[2], x[3]);
+            }
+        }
     }
 }
 
 // leaf value = mean over the 48 rivers of the subgames' root values (0 where the river card
-// is in the hand)
+// is in the hand); one CTA per (leaf, half of the hands), a hand per thread, whose 48 pairs of dependent
+// loads go eight at a time
+constexpr int kGatherThreads = 672;
 template <typename T>
-__global__ void __launch_bounds__(FT) gather_kernel(const BPack *__restrict__ packs, const T *__restrict__ root,
+__global__ void __launch_bounds__(kGatherThreads) gather_kernel(const BPack *__restrict__ packs, const T *__restrict__ root,
                                                      const int *__restrict__ slot_node, const FNode *__restrict__ nodes,
                                                      T *__restrict__ leafV) {
     const int j = blockIdx.x;
+    const int h = blockIdx.y * kGatherThreads + threadIdx.x;
+    if (h >= kH) return;
     T *out = leafV + (size_t)nodes[slot_node[j]].edge * kH;
-    for (int h = threadIdx.x; h < kH; h += FT) {
-        T s = T(0);
-        for (int k = 0; k < kRivers; k++) {
-            const int sg = j * kRivers + k;
-            const int p = packs[sg].pos_of[h];
-            if (p != 0xFFFF) s += root[(size_t)sg * kBRow + p];
-        }
-        out[h] = s / T(kRivers);
+    T s = T(0);
+#pragma unroll 1
+    for (int k = 0; k < kRivers; k += 8) {
+        int p[8];
+        T x[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) p[i] = packs[j * kRivers + k + i].pos_of[h];
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = p[i] != 0xFFFF ? root[(size_t)(j * kRivers + k + i) * kBRow + p[i]] : T(0);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (p[i] != 0xFFFF) s += x[i];
     }
+    out[h] = s / T(kRivers);
 }
 
 // ---- net leaves ----
@@ -396,7 +444,7 @@ struct Game {
     template <typename T>
     int down(T *R, const float *src, int average) {
         for (int l = 0; l + 1 < (int)levels.size(); l++) {
-            if (level_size(l)) down_kernel<T><<<level_size(l), FT, 0, stream>>>(fview(), level_ptr(l), R, src, average);
+            if (level_size(l)) down_kernel<T><<<dim3(level_size(l), kHandChunks), FT, 0, stream>>>(fview(), level_ptr(l), R, src, average);
             if (deal_size(l)) deal_down_kernel<T><<<dim3(deal_size(l), 52), FT, 0, stream>>>(fview(), deal_ptr(l), R);
         }
         cudaError_t e = cudaGetLastError();
@@ -407,9 +455,9 @@ struct Game {
     int up(int upd, const T *R, T *V, const T *leafV, const float *src, int average) {
         for (int l = (int)levels.size() - 1; l >= 0; l--) {
             if (deal_size(l))
-                deal_up_kernel<T><<<dim3(deal_size(l), (kH + FT - 1) / FT), FT, 0, stream>>>(fview(), deal_ptr(l), V);
+                deal_up_kernel<T><<<dim3(deal_size(l), kHandChunks), FT, 0, stream>>>(fview(), deal_ptr(l), V);
             if (!level_size(l)) continue;
-            up_kernel<T, MODE><<<level_size(l), FT, 0, stream>>>(fview(), level_ptr(l), upd, R, V, leafV,
+            up_kernel<T, MODE><<<dim3(level_size(l), kHandChunks), FT, 0, stream>>>(fview(), level_ptr(l), upd, R, V, leafV,
                                                                  MODE == kUpCFR ? d_reg : nullptr,
                                                                  MODE == kUpCFR ? d_avg : nullptr, src, average,
                                                                  d_wt);
@@ -424,12 +472,12 @@ struct Game {
         if (!batch[b]) return 0;
         const BatchView &v = view[b];
         const bool f64 = sizeof(T) == 8;
-        scatter_kernel<T><<<v.count, FT, 0, stream>>>(v.packs, R, d_slots[b],
+        scatter_kernel<T><<<v.count / kScatterRivers, FT, 0, stream>>>(v.packs, R, d_slots[b],
                                                       f64 ? (T *)v.ranges64 : (T *)v.ranges);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return ffail("range scatter", e);
         if (int st = batch_run_pass(batch[b], mode, player, f64 ? 1 : 0, use_average, d_root[b], stream)) return st;
-        gather_kernel<T><<<(int)slots[b].size(), FT, 0, stream>>>(v.packs, (const T *)d_root[b], d_slots[b], d_nodes,
+        gather_kernel<T><<<dim3((int)slots[b].size(), 2), kGatherThreads, 0, stream>>>(v.packs, (const T *)d_root[b], d_slots[b], d_nodes,
                                                                   leafV);
         e = cudaGetLastError();
         return e == cudaSuccess ? 0 : ffail("value gather", e);
@@ -515,7 +563,7 @@ int full_exploitability(Game *g, int resolve_iterations, double *br0, double *br
     if (resolve_iterations > 0 && g->batch[0]) {
         if (int st = g->down<float>(g->d_R, g->d_avg, 1)) return st;
         const BatchView &v = g->view[0];
-        scatter_kernel<float><<<v.count, FT, 0, g->stream>>>(v.packs, g->d_R, g->d_slots[0], v.ranges);
+        scatter_kernel<float><<<v.count / kScatterRivers, FT, 0, g->stream>>>(v.packs, g->d_R, g->d_slots[0], v.ranges);
         if (int st = batch_clear(g->batch[0], g->stream)) return st;
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
