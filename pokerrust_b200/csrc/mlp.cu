@@ -139,6 +139,34 @@ struct EpiBiasF32 {  // Y = acc + b (f32)
         }
     }
 };
+struct EpiBiasOut {  // out = acc + b (f32) on live rows and columns, rows of kOut values
+    const float *bias;
+    float *out;
+    int count, aligned;
+    template <class R, class P>
+    __device__ void operator()(R const &reg, P const &pos, int m0, int n0, int) const {
+        int mr, nr;
+        static_assert(kOut % 4 == 0, "whole quads");
+        if (aligned && cute::size(reg) == 32 && row_run(pos, &mr, &nr)) {
+            const int m = m0 + mr, n = n0 + nr;
+            if (m >= count) return;
+            float4 *o = reinterpret_cast<float4 *>(out + (size_t)m * kOut + n);
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                if (n + 4 * q >= kOut) break;
+                const float4 bq = *reinterpret_cast<const float4 *>(bias + n + 4 * q);
+                o[q] = make_float4(reg(4 * q) + bq.x, reg(4 * q + 1) + bq.y, reg(4 * q + 2) + bq.z,
+                                   reg(4 * q + 3) + bq.w);
+            }
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < cute::size(reg); i++) {
+            const int m = m0 + cute::get<0>(pos(i)), n = n0 + cute::get<1>(pos(i));
+            if (m < count && n < kOut) out[(size_t)m * kOut + n] = reg(i) + bias[n];
+        }
+    }
+};
 struct EpiGeluGrad {  // dZ = acc * gelu'(Z), bf16
     const bf16 *Z;
     bf16 *dZ;
@@ -355,12 +383,6 @@ __global__ void to_bf16_kernel(const float *__restrict__ w, bf16 *__restrict__ w
         wb[i] = bf16(w[i]);
 }
 
-__global__ void copy_out_kernel(const float *__restrict__ Y, float *__restrict__ out, int n) {
-    const int m = blockIdx.x;
-    if (m >= n) return;
-    for (int j = threadIdx.x; j < kOut; j += blockDim.x) out[(size_t)m * kOut + j] = Y[(size_t)m * kOutPad + j];
-}
-
 struct Net {
     int rows = 0;  // batch rows (multiple of 256)
     cudaStream_t stream = nullptr;
@@ -388,7 +410,22 @@ struct Net {
         if (persistent) return gemm::run_persistent<128, MA, MB>(A, B, M, N, K, epi, d_err, stream, splits);
         return gemm::run<BN, MA, MB>(A, B, M, N, K, epi, d_err, stream, splits);
     }
+    // A forward GEMM over M rows, with the widest tile that still gives every SM one: over few rows the
+    // pass is a chain of five launches that leave most SMs idle, and narrower tiles shorten each CTA's
+    // copies and epilogue. (The sums run over K in the same order for every width.) A forward call of 128
+    // and 900 samples takes 87 and 101 us so, 99 and 113 with tiles of 128 columns throughout, 194 and 193
+    // with 256 columns over all 4,096 rows.
+    template <class Epi>
+    cudaError_t mm_rows(const bf16 *A, const bf16 *B, int M, int N, int K, Epi epi) {
+        const int rows_m = M / gemm::kBM;
+        if (persistent || rows_m * (N / 128) > sms) return mm<256>(A, B, M, N, K, epi);
+        if (rows_m * (N / 64) > sms) return mm<128>(A, B, M, N, K, epi);
+        return mm<64>(A, B, M, N, K, epi);
+    }
     std::vector<void *> owned;
+    int sms = 148;
+    int *h_err = nullptr;  // pinned
+    double *h_partial = nullptr;
 
     template <class T>
     bool alloc(T **p, size_t n) {
@@ -399,6 +436,8 @@ struct Net {
     ~Net() {
         if (stream) cudaStreamSynchronize(stream);
         for (void *p : owned) cudaFree(p);
+        cudaFreeHost(h_err);
+        cudaFreeHost(h_partial);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -408,18 +447,22 @@ struct Net {
         return e == cudaErrorInvalidValue ? 2 : 1;
     }
 
-    // forward pass over X (rows), Y = output pre-loss (f32)
-    int forward() {
+    // forward pass over the first M rows of X (a multiple of 128): the output to Y (f32), or the live
+    // part of the first `count` rows to `out`
+    int forward(int M, float *out = nullptr, int count = 0) {
         cudaError_t e = cudaSuccess;
         const bf16 *in = X;
         for (int l = 0; l < 4 && e == cudaSuccess; l++) {
             EpiBiasGelu epi{b[l], Z[l], H[l], kN[l]};
-            e = mm<256>(in, Wb[l], rows, kN[l], kK[l], epi);
+            e = mm_rows(in, Wb[l], M, kN[l], kK[l], epi);
             in = H[l];
         }
-        if (e == cudaSuccess) {
+        if (e == cudaSuccess && out) {
+            EpiBiasOut epi{b[4], out, count, (reinterpret_cast<uintptr_t>(out) & 15) == 0};
+            e = mm_rows(in, Wb[4], M, kOutPad, kHid, epi);
+        } else if (e == cudaSuccess) {
             EpiBiasF32 epi{b[4], Y, kOutPad};
-            e = mm<256>(in, Wb[4], rows, kOutPad, kHid, epi);
+            e = mm_rows(in, Wb[4], M, kOutPad, kHid, epi);
         }
         return check(e, "forward");
     }
@@ -518,6 +561,12 @@ void *pr_mlp_new(int rows, uint64_t seed) {
     ok = ok && n->alloc(&n->X, (size_t)rows * kInPad) && n->alloc(&n->Y, (size_t)rows * kOutPad) &&
          n->alloc(&n->dY, (size_t)rows * kOutPad) && n->alloc(&n->partial, rows) &&
          n->alloc(&n->bias_parts, (size_t)kBiasChunks * kOutPad);
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n->sms <= 0)
+        n->sms = 148;
+    ok = ok && cudaMallocHost((void **)&n->h_err, sizeof(int)) == cudaSuccess &&
+         cudaMallocHost((void **)&n->h_partial, sizeof(double) * rows) == cudaSuccess;
     for (int l = 0; l < kLayers && ok; l++) ok = n->alloc(&n->parts[l], (size_t)Net::kSplits * kN[l] * kK[l]);
     for (int l = 0; l < 4 && ok; l++)
         ok = n->alloc(&n->Z[l], (size_t)rows * kHid) && n->alloc(&n->H[l], (size_t)rows * kHid) &&
@@ -566,18 +615,17 @@ int pr_mlp_set_persistent(void *net, int on) {
 }
 
 namespace {
-int load_inputs(Net *n, const float *ranges, const unsigned long long *boards, const float *scalars, int count) {
-    if (count < 1 || count > n->rows) return 2;
-    assemble_kernel<<<n->rows, 256, 0, n->stream>>>(ranges, boards, scalars, n->X, count);
+// rows [0, M) of X, of which the first `count` are inputs and the others zero
+int load_inputs(Net *n, const float *ranges, const unsigned long long *boards, const float *scalars, int count, int M) {
+    assemble_kernel<<<M, 256, 0, n->stream>>>(ranges, boards, scalars, n->X, count);
     return n->check(cudaGetLastError(), "inputs");
 }
 int finish(Net *n) {
-    int err = 0;
-    cudaError_t e = cudaStreamSynchronize(n->stream);
-    if (e == cudaSuccess) e = cudaMemcpy(&err, n->d_err, sizeof(int), cudaMemcpyDeviceToHost);
+    cudaError_t e = cudaMemcpyAsync(n->h_err, n->d_err, sizeof(int), cudaMemcpyDeviceToHost, n->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(n->stream);
     if (e != cudaSuccess) return n->check(e, "pass");
-    if (err) {
-        fprintf(stderr, "pokerrust_b200: value network: a GEMM wait timed out (bits %d)\n", err);
+    if (*n->h_err) {
+        fprintf(stderr, "pokerrust_b200: value network: a GEMM wait timed out (bits %d)\n", *n->h_err);
         return 1;
     }
     return 0;
@@ -591,9 +639,11 @@ int pr_mlp_forward(void *net, const float *ranges, const uint64_t *boards, const
     prb::TraceRange trace("value network forward");
     Net *n = (Net *)net;
     if (!n || !ranges || !boards || !scalars || !out) return 2;
-    if (int st = load_inputs(n, ranges, (const unsigned long long *)boards, scalars, count)) return st;
-    if (int st = n->forward()) return st;
-    copy_out_kernel<<<count, 256, 0, n->stream>>>(n->Y, out, count);
+    if (count < 1 || count > n->rows) return 2;
+    // only the row tiles that hold samples (see mm_rows for what that gives)
+    const int M = (count + prb::gemm::kBM - 1) / prb::gemm::kBM * prb::gemm::kBM;
+    if (int st = load_inputs(n, ranges, (const unsigned long long *)boards, scalars, count, M)) return st;
+    if (int st = n->forward(M, out, count)) return st;
     return finish(n);
 }
 
@@ -604,18 +654,22 @@ int pr_mlp_train_step(void *net, const float *ranges, const uint64_t *boards, co
     prb::TraceRange trace("value network training step");
     Net *n = (Net *)net;
     if (!n || !ranges || !boards || !scalars || !targets) return 2;
-    if (int st = load_inputs(n, ranges, (const unsigned long long *)boards, scalars, count)) return st;
-    if (int st = n->forward()) return st;
+    if (count < 1 || count > n->rows) return 2;
+    if (int st = load_inputs(n, ranges, (const unsigned long long *)boards, scalars, count, n->rows)) return st;
+    if (int st = n->forward(n->rows)) return st;
     loss_kernel<<<n->rows, 256, 0, n->stream>>>(n->Y, targets, n->dY, n->partial, count, n->rows);
     if (int st = n->backward()) return st;
     if (lr > 0.0f)
         if (int st = n->adam(lr)) return st;
+    if (loss) {
+        const cudaError_t e =
+            cudaMemcpyAsync(n->h_partial, n->partial, sizeof(double) * count, cudaMemcpyDeviceToHost, n->stream);
+        if (e != cudaSuccess) return n->check(e, "loss");
+    }
     if (int st = finish(n)) return st;
     if (loss) {
-        std::vector<double> p(n->rows);
-        cudaMemcpy(p.data(), n->partial, sizeof(double) * n->rows, cudaMemcpyDeviceToHost);
         double s = 0;
-        for (int i = 0; i < count; i++) s += p[i];
+        for (int i = 0; i < count; i++) s += n->h_partial[i];
         *loss = s / ((double)count * kOut);
     }
     return 0;
