@@ -188,6 +188,10 @@ struct RiverPart {
 };
 
 __device__ __forceinline__ void bar_rank_list() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// The last warp has added the staged runs of the river card before (arrive); warp 0 waits for that
+// before it adds the blocked hands' term to bucket 0, which those runs share.
+__device__ __forceinline__ void bar_staged_arrive() { asm volatile("bar.arrive 2, 64;" ::: "memory"); }
+__device__ __forceinline__ void bar_staged_wait() { asm volatile("bar.sync 2, 64;" ::: "memory"); }
 
 // Loads n consecutive values (n a multiple of 4 floats / 2 doubles) with 16-byte loads.
 __device__ __forceinline__ void load_row(const float *p, float *o, int n) {
@@ -493,7 +497,7 @@ __global__ void __launch_bounds__(NT, 1)
     // ---- the 48 river cards ----
     const int per_cta = SPLIT ? 48 / splits : 48;
     const int first_river = SPLIT ? blockIdx.x % splits * per_cta : 0;
-    int rc_done = 0, nth = -1;
+    int nth = -1;  // river cards before this one
     for (int rc = 0; rc < 52; rc++) {
         const unsigned long long rb = 1ull << rc;
         if (rb & d.board4) continue;
@@ -504,9 +508,12 @@ __global__ void __launch_bounds__(NT, 1)
         const BoardPack *__restrict__ pk = packs + slot;
         __syncthreads();  // previous river's readers are done with Pg, VC, Cf, Tf
         if constexpr (MODE == kModeCFR) {
-            if (!SPLIT && warp == NT / 32 - 1 && lane < ACC && rc_done > 0) resolve_stage(S, lane);
+            if (!SPLIT && warp == NT / 32 - 1 && nth > 0) {
+                if (lane < ACC) resolve_stage(S, lane);
+                __syncwarp();
+                bar_staged_arrive();
+            }
         }
-        rc_done++;
 
         if (warp < 4) {
             // rank list: lane g holds slots [9g, 9g + 9); writes the prefix sum at every
@@ -579,14 +586,9 @@ __global__ void __launch_bounds__(NT, 1)
                 }
 #pragma unroll
                 for (int f = 0; f < kNumFold; f++) S.Tf[f] = total[fold_channel(f, UPD)];
-                if constexpr (MODE == kModeCFR) {
-                    // blocked hands' contribution to bucket 0 (see the file comment)
+                if constexpr (SPLIT && MODE == kModeCFR) {
 #pragma unroll
-                    for (int c = 0; c < kNumLeaves; c++) {
-                        const float t = total[leaf_channel(c, UPD)];
-                        if constexpr (SPLIT) part->total[c] = t;
-                        else S.abar[0][c] = __fmaf_rn(c < kNumSD ? -235.0f : 235.0f, t, S.abar[0][c]);
-                    }
+                    for (int c = 0; c < kNumLeaves; c++) part->total[c] = total[leaf_channel(c, UPD)];
                 }
             }
             // W - B of every tie group: prefix at its start + prefix at its end - total
@@ -594,6 +596,18 @@ __global__ void __launch_bounds__(NT, 1)
             for (int gg = g; gg < G; gg += 128) {
 #pragma unroll
                 for (int c = 0; c < kNumSD; c++) S.VG[gg][c] = S.Pg[gg][c] + S.Pg[gg + 1][c] - total[c];
+            }
+            if constexpr (!SPLIT && MODE == kModeCFR) {
+                // blocked hands' contribution to bucket 0 (see the file comment)
+                if (warp == 0 && nth > 0) {
+                    __syncwarp();
+                    bar_staged_wait();
+                }
+                if (tid == 0) {
+#pragma unroll
+                    for (int c = 0; c < kNumLeaves; c++)
+                        S.abar[0][c] = __fmaf_rn(c < kNumSD ? -235.0f : 235.0f, total[leaf_channel(c, UPD)], S.abar[0][c]);
+                }
             }
         } else {
             // card lists: 8 lanes per list, 6 slots per lane, 4 lists per warp. Each group of
