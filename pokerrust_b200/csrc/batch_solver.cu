@@ -228,8 +228,9 @@ static_assert(sizeof(PackWords) == offsetof(BPack, pos_of) - offsetof(BPack, clp
 template <typename V>
 struct Job {
     int x0;         // the scanned leaf's row in X, in values
-    int show;       // it is a showdown
-    V stake, fold;  // signed stakes of the scanned leaf and of the fold before it (0: none)
+    uint16_t show;  // it is a showdown
+    uint16_t pair;  // ... and the row before it is a fold of the job
+    V stake, fold;  // signed stakes of the scanned leaf and of that fold (either may be zero)
 };
 constexpr int kMaxGroupLeaves = 32;  // leaves of a group: a warp lays out its jobs
 
@@ -391,6 +392,7 @@ __device__ __forceinline__ int lay_out_jobs(const Smem<V> &S, int g0, int g1, in
         Job<V> &job = S.job[__popc(starts & ((1u << lane) - 1))];
         job.x0 = (lane + (pair ? 1 : 0)) * kBRow;
         job.show = pair || ln.kind == kBShowdown;
+        job.pair = pair;
         job.stake = pair ? V(next_stake) : ln.kind == kBFold && ln.actor == p ? -V(ln.stake) : V(ln.stake);
         job.fold = pair ? -V(ln.stake) : V(0);
     }
@@ -528,7 +530,7 @@ __device__ __forceinline__ void leaf_values(const Smem<V> &S, const BPack *__res
                     val[k] = pos0 + k < kBLive ? mul(job.stake, (vg - v1) - v2) : V(0);
                 }
             }
-            if (!job.show || job.fold != V(0)) {
+            if (!job.show || job.pair) {
                 V xv[K], fold[K];
                 ld_k<K>(x, pos0, xv);
                 const V T = S.T[q], m = job.show ? job.fold : job.stake;
