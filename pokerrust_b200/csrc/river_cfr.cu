@@ -406,8 +406,9 @@ __device__ __forceinline__ void update_bucket(int b, float (&reg)[kEdges], const
     }
 }
 
-// SPLIT: `splits` CTAs share a root, each with 48 / splits of its river cards, and leave their sums to
-// finish_kernel: the values in outs [root][split][hand], the bucket sums in parts [root][river card].
+// SPLIT: `splits` CTAs share a root, each with 48 / splits of its river cards, and leave every card's
+// values (outs [root][river card][hand]) and bucket sums (parts [root][river card]) to finish_kernel, which
+// adds them in river order: results do not depend on the number of CTAs.
 template <int MODE, typename V, bool AVG, int UPD, bool SPLIT>
 __global__ void __launch_bounds__(NT, 1)
     river_kernel(const SubgameDesc *__restrict__ desc, const V *__restrict__ ranges, V *__restrict__ results,
@@ -855,9 +856,16 @@ __global__ void __launch_bounds__(NT, 1)
                 }
             }
         }
-        if constexpr (SPLIT && MODE == kModeCFR) {
-            // this river card's bucket sums leave; the accumulators start at zero for the next one
+        if constexpr (SPLIT) {
+            // this river card's values leave, then its bucket sums; both start at zero for the next one
             __syncthreads();
+            V *to = outs + ((size_t)sg * 48 + nth) * kRangeStride;
+            for (int i = tid; i < kRangeStride; i += NT) {
+                to[i] = S.out[i];
+                S.out[i] = V(0);
+            }
+        }
+        if constexpr (SPLIT && MODE == kModeCFR) {
             const int *key = &S.stage_key[0][0];
             const float *stage = &S.stage[0][0][0];
             uint8_t *first = reinterpret_cast<uint8_t *>(S.Pg);  // first staged run of each bucket
@@ -888,11 +896,8 @@ __global__ void __launch_bounds__(NT, 1)
             }
         }
     }
+    if constexpr (SPLIT) return;
     __syncthreads();
-    if constexpr (SPLIT) {
-        for (int i = tid; i < kRangeStride; i += NT) outs[(size_t)blockIdx.x * kRangeStride + i] = S.out[i];
-        return;
-    }
     if constexpr (MODE == kModeCFR) {
         if (warp == NT / 32 - 1 && lane < ACC) resolve_stage(S, lane);
         __syncthreads();
@@ -924,9 +929,8 @@ constexpr int kFinBuckets = 16;
 constexpr int kFinThreads = kFinBuckets * 18 + 32;
 template <int MODE, typename V, bool AVG, int UPD>
 __global__ void __launch_bounds__(kFinThreads)
-    finish_kernel(const SubgameDesc *__restrict__ desc, const V *__restrict__ outs, int splits,
-                  const void *__restrict__ parts, V *__restrict__ results, float *__restrict__ regrets,
-                  float *__restrict__ avg_sums) {
+    finish_kernel(const SubgameDesc *__restrict__ desc, const V *__restrict__ outs, const void *__restrict__ parts,
+                  V *__restrict__ results, float *__restrict__ regrets, float *__restrict__ avg_sums) {
     constexpr int ACC = kNumLeaves + (AVG ? 1 : 0);
     const int sg = blockIdx.x, tid = threadIdx.x;
     if constexpr (MODE == kModeCFR) {
@@ -982,7 +986,8 @@ __global__ void __launch_bounds__(kFinThreads)
     for (int i = tid; i < kShare; i += kFinBuckets * 18) {
         const int h = blockIdx.y * kShare + i;
         V sum = V(0);
-        for (int q = 0; q < splits; q++) sum += outs[((size_t)sg * splits + q) * kRangeStride + h];
+#pragma unroll 16
+        for (int q = 0; q < 48; q++) sum += outs[((size_t)sg * 48 + q) * kRangeStride + h];
         results[(size_t)sg * kRangeStride + h] = h < kHands ? sum * (V(1) / V(48)) : V(0);
     }
 }
@@ -1027,7 +1032,7 @@ cudaError_t launch_upd(const SubgameDesc *desc, int n, const V *ranges, V *resul
     if (L.total > 227u * 1024u) return cudaErrorInvalidConfiguration;
     const int splits = scratch ? pick_splits(n, sm_count(), MODE == kModeCFR) : 1;
     if (splits > 1) {
-        const size_t outs = aligned((size_t)n * splits * kRangeStride * sizeof(V));
+        const size_t outs = aligned((size_t)n * 48 * kRangeStride * sizeof(V));
         const size_t parts = MODE == kModeCFR ? (size_t)n * 48 * sizeof(RiverPart<ACC>) : 0;
         unsigned char *mem = static_cast<unsigned char *>(scratch->take(outs + parts, stream));
         if (mem) {
@@ -1049,7 +1054,7 @@ cudaError_t launch_upd(const SubgameDesc *desc, int n, const V *ranges, V *resul
                 cfg.numAttrs = 1;
                 if (e == cudaSuccess)
                     e = cudaLaunchKernelEx(&cfg, finish_kernel<MODE, V, AVG, UPD>, desc, reinterpret_cast<const V *>(mem),
-                                           splits, (const void *)(mem + outs), results, regrets, avg);
+                                           (const void *)(mem + outs), results, regrets, avg);
             }
             scratch->give_back(mem, stream);
             return e;

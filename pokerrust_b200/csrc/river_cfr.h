@@ -32,7 +32,7 @@ size_t river_smem_bytes(int mode, int fp64, int max_groups, int max_card_groups)
 // read only). ranges / results: n rows of kRangeStride values; regrets: n * 26 * 256.
 // In CFR mode with own_ranges (the updater's ranges, same rows) and avg_sums (n * 26 * 256)
 // the pass also accumulates average-strategy sums. With `scratch`, passes over few roots spread each
-// root's river cards over several CTAs (same bucket sums and regrets, bit for bit).
+// root's river cards over several CTAs (same values, bucket sums and regrets, bit for bit).
 cudaError_t launch_river(int mode, const SubgameDesc *desc, int n, const float *ranges, float *results,
                          float *regrets, const BoardPack *packs, unsigned long long flop, int updater,
                          int max_groups, int max_card_groups, const float *own_ranges, float *avg_sums,
