@@ -1081,6 +1081,16 @@ cudaError_t launch_one(const SubgameDesc *desc, int n, const V *ranges, V *resul
 
 }  // namespace
 
+namespace {
+// Making or growing a pool is a call that would end a capture another stream or thread has under way (in
+// the global mode); this thread's calls are exempt while one of these is in scope.
+struct BesideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+}  // namespace
+
 void *RiverScratch::take(size_t bytes, cudaStream_t stream) {
     // an allocation inside a capture would become part of the caller's graph
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -1088,6 +1098,7 @@ void *RiverScratch::take(size_t bytes, cudaStream_t stream) {
         cudaGetLastError();
         return nullptr;
     }
+    const BesideCaptures relaxed;
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!pool) {
@@ -1111,7 +1122,10 @@ void *RiverScratch::take(size_t bytes, cudaStream_t stream) {
     return p;
 }
 
-void RiverScratch::give_back(void *p, cudaStream_t stream) { cudaFreeAsync(p, stream); }
+void RiverScratch::give_back(void *p, cudaStream_t stream) {
+    const BesideCaptures relaxed;
+    cudaFreeAsync(p, stream);
+}
 
 RiverScratch::~RiverScratch() {
     if (pool) cudaMemPoolDestroy(pool);
