@@ -36,6 +36,9 @@
 // counts of the flop's boards (BoardPack::num_groups / num_card_groups).
 #include <cuda_runtime.h>
 
+#include <map>
+#include <mutex>
+
 #include "device_common.cuh"
 #include "layout.h"
 #include "river_cfr.h"
@@ -1089,7 +1092,48 @@ struct BesideCaptures {
     BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
     ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
+
+// The pool of each device and the RiverScratch that draw on it. (Not destroyed at exit: a builder may be
+// freed later.)
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    int users = 0;
+};
+std::mutex g_pools_mu;
+std::map<int, DevicePool> &pools() {
+    static auto *m = new std::map<int, DevicePool>;
+    return *m;
+}
 }  // namespace
+
+bool RiverScratch::attach() {
+    std::lock_guard<std::mutex> lk(g_pools_mu);
+    if (pool) return true;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    if (cudaGetDevice(&props.location.id) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    DevicePool &d = pools()[props.location.id];
+    if (!d.pool) {
+        if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) {
+            d.pool = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        unsigned long long keep = kMaxScratch;
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        // passes of builders on several streams do not wait for one another's memory
+        int wait = 0;
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolReuseAllowInternalDependencies, &wait);
+    }
+    d.users++;
+    device = props.location.id;
+    pool = d.pool;
+    return true;
+}
 
 void *RiverScratch::take(size_t bytes, cudaStream_t stream) {
     // an allocation inside a capture would become part of the caller's graph
@@ -1099,21 +1143,7 @@ void *RiverScratch::take(size_t bytes, cudaStream_t stream) {
         return nullptr;
     }
     const BesideCaptures relaxed;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!pool) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-                pool = nullptr;
-                cudaGetLastError();
-                return nullptr;
-            }
-            unsigned long long keep = kMaxScratch;
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        }
-    }
+    if (!pool && !attach()) return nullptr;
     void *p = nullptr;
     if (cudaMallocFromPoolAsync(&p, bytes, pool, stream) != cudaSuccess) {
         cudaGetLastError();
@@ -1128,7 +1158,12 @@ void RiverScratch::give_back(void *p, cudaStream_t stream) {
 }
 
 RiverScratch::~RiverScratch() {
-    if (pool) cudaMemPoolDestroy(pool);
+    std::lock_guard<std::mutex> lk(g_pools_mu);
+    if (!pool) return;
+    DevicePool &d = pools()[device];
+    if (--d.users > 0) return;
+    cudaMemPoolDestroy(d.pool);
+    d.pool = nullptr;
 }
 
 size_t river_smem_bytes(int mode, int fp64, int max_groups, int max_card_groups) {

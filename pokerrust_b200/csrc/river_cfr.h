@@ -2,7 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include <mutex>
+#include <atomic>
 
 #include "layout.h"
 
@@ -10,14 +10,16 @@ namespace prb {
 
 enum { kModeCFR = 0, kModeBR = 1 };
 
-// Device memory of split passes (few roots: see launch_river), taken and given back in stream order
-// from a pool of its own, so that passes on several streams and threads do not share it. The pool keeps
-// at most kMaxScratch bytes between passes and goes with its owner. No memory is handed out while the
-// stream is capturing: those passes run unsplit.
+// Device memory of split passes (few roots: see launch_river), taken and given back in stream order, so
+// that passes on several streams and threads do not share it. It comes from one pool per device, which
+// keeps at most kMaxScratch bytes between passes, whatever the number of builders, and goes with the last
+// of those that drew on it. No memory is handed out while the stream is capturing: those passes run
+// unsplit.
 struct RiverScratch {
     static constexpr size_t kMaxScratch = (size_t)256 << 20;
-    std::mutex mu;
-    cudaMemPool_t pool = nullptr;
+    int device = 0;
+    std::atomic<cudaMemPool_t> pool{nullptr};
+    bool attach();
     void *take(size_t bytes, cudaStream_t stream);
     void give_back(void *p, cudaStream_t stream);
     ~RiverScratch();

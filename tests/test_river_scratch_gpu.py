@@ -1,5 +1,6 @@
-"""Device memory that passes over few roots take for themselves: taking it does not stand in the way of a
-stream that is being captured elsewhere."""
+"""Device memory that passes over few roots take for themselves: one bounded pool per device, whatever
+the number of builders, given back with the last of them; and none of it stands in the way of a stream
+that is being captured elsewhere."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -14,6 +15,33 @@ def _builder(P, n):
         b.add(FLOP | (1 << TURNS[i % len(TURNS)]), 2.0 + i)
     b.regrets()  # device state is in place
     return b
+
+
+def test_many_builders_hold_one_pool():
+    import torch
+
+    import pokerrust_b200 as P
+    tables = P.build_flop_tables(FLOP)
+    n = 70
+    builders = [_builder(P, n) for _ in range(8)]
+    d_in = torch.rand((n, 1328), device="cuda")
+    d_out = torch.zeros((n, 1328), device="cuda")
+
+    def held():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    free = held()
+    for b in builders:
+        b.evaluate_device(tables, 0, False, d_in.data_ptr(), d_out.data_ptr())
+    used = free - held()
+    # a pass over 70 roots takes more than 64 MB, the pool keeps 256 MB at most (64 MB to spare for the
+    # kernels, loaded on first use)
+    assert 64 << 20 < used <= 320 << 20, used >> 20
+    for b in builders:
+        b.close()
+    assert held() >= free
+    P.free_eval(tables)
 
 
 def test_first_pass_beside_a_capture():
@@ -41,6 +69,6 @@ def test_first_pass_beside_a_capture():
             torch.cuda.synchronize()
             assert (y == 2).all()
         torch.cuda.synchronize()
-        b.close()
+        b.close()  # and with it the pool
     assert torch.equal(*d_out)
     P.free_eval(tables)
