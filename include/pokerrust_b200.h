@@ -102,6 +102,10 @@ int pr_set_average(void *builder, const float *in);
 int pr_builder_count(void *builder);
 int pr_range_stride(void);
 
+/* CTAs that each root's river cards were spread over in the builder's last pass (1: one CTA per
+ * root, 0: no pass yet). Results do not depend on it. */
+int pr_builder_splits(void *builder);
+
 /* Bucket regrets, count * 26 * 256 floats in the reference's edge order
  * (src/cuda/builder.cu:85-97 numbering). Host buffers; synchronous. */
 int pr_get_regrets(void *builder, float *out);

@@ -704,6 +704,8 @@ int pr_set_average(void *builder, const float *in) {
 
 int pr_builder_count(void *builder) { return builder ? (int)((Builder *)builder)->desc.size() : 0; }
 
+int pr_builder_splits(void *builder) { return builder ? ((Builder *)builder)->scratch.splits.load() : 0; }
+
 int pr_range_stride(void) { return kRangeStride; }
 
 int pr_get_regrets(void *builder, float *out) {

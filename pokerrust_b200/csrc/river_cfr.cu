@@ -1039,6 +1039,7 @@ cudaError_t launch_upd(const SubgameDesc *desc, int n, const V *ranges, V *resul
         const size_t parts = MODE == kModeCFR ? (size_t)n * 48 * sizeof(RiverPart<ACC>) : 0;
         unsigned char *mem = static_cast<unsigned char *>(scratch->take(outs + parts, stream));
         if (mem) {
+            scratch->splits = splits;
             auto kernel = river_kernel<MODE, V, AVG, UPD, true>;
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
             if (e == cudaSuccess) {
@@ -1063,6 +1064,7 @@ cudaError_t launch_upd(const SubgameDesc *desc, int n, const V *ranges, V *resul
             return e;
         }
     }
+    if (scratch) scratch->splits = 1;
     auto kernel = river_kernel<MODE, V, AVG, UPD, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
     if (e != cudaSuccess) return e;

@@ -18,6 +18,7 @@ enum { kModeCFR = 0, kModeBR = 1 };
 struct RiverScratch {
     static constexpr size_t kMaxScratch = (size_t)256 << 20;
     int device = 0;
+    std::atomic<int> splits{0};  // CTAs per root of the last pass, 0 before the first
     std::atomic<cudaMemPool_t> pool{nullptr};
     bool attach();
     void *take(size_t bytes, cudaStream_t stream);

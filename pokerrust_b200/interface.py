@@ -90,6 +90,8 @@ def lib():
         L.pr_download_batch.argtypes = [vp, i32, i32, vp]
         L.pr_builder_count.restype = i32
         L.pr_builder_count.argtypes = [vp]
+        L.pr_builder_splits.restype = i32
+        L.pr_builder_splits.argtypes = [vp]
         L.pr_range_stride.restype = i32
         L.pr_get_regrets.restype = i32
         L.pr_get_regrets.argtypes = [vp, vp]
@@ -402,6 +404,11 @@ class Builder:
     @property
     def count(self):
         return lib().pr_builder_count(self.ptr)
+
+    @property
+    def splits(self):
+        """CTAs per root of the last pass (0 before the first)."""
+        return lib().pr_builder_splits(self.ptr)
 
     def upload_all(self, ranges):
         ranges = np.ascontiguousarray(ranges, dtype=np.float32)
