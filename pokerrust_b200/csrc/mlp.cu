@@ -461,8 +461,8 @@ struct Net {
     }
     std::vector<void *> owned;
     int sms = 148;
-    int *h_err = nullptr;  // pinned
-    double *h_partial = nullptr;
+    double *h_partial = nullptr;  // pinned, with h_err behind it (a pinned allocation takes a millisecond)
+    int *h_err = nullptr;
 
     template <class T>
     bool alloc(T **p, size_t n) {
@@ -474,7 +474,6 @@ struct Net {
         if (stream) cudaStreamSynchronize(stream);
         if (side) cudaStreamSynchronize(side);
         for (void *p : owned) cudaFree(p);
-        cudaFreeHost(h_err);
         cudaFreeHost(h_partial);
         for (cudaEvent_t ev : ready)
             if (ev) cudaEventDestroy(ev);
@@ -625,8 +624,8 @@ void *pr_mlp_new(int rows, uint64_t seed) {
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n->sms <= 0)
         n->sms = 148;
-    ok = ok && cudaMallocHost((void **)&n->h_err, sizeof(int)) == cudaSuccess &&
-         cudaMallocHost((void **)&n->h_partial, sizeof(double) * rows) == cudaSuccess;
+    ok = ok && cudaMallocHost((void **)&n->h_partial, sizeof(double) * rows + sizeof(int)) == cudaSuccess;
+    n->h_err = reinterpret_cast<int *>(n->h_partial + rows);
     for (int l = 0; l < kLayers && ok; l++) ok = n->alloc(&n->parts[l], (size_t)Net::kSplits * kN[l] * kK[l]);
     for (int l = 0; l < 4 && ok; l++)
         ok = n->alloc(&n->Z[l], (size_t)rows * kHid) && n->alloc(&n->H[l], (size_t)rows * kHid) &&
