@@ -447,11 +447,13 @@ struct Net {
         if (persistent) return gemm::run_persistent<128, MA, MB>(A, B, M, N, K, epi, d_err, on, splits);
         return gemm::run<BN, MA, MB>(A, B, M, N, K, epi, d_err, on, splits);
     }
-    // A forward GEMM over M rows, with the widest tile that still gives every SM one: over few rows the
-    // pass is a chain of five launches that leave most SMs idle, and narrower tiles shorten each CTA's
-    // copies and epilogue. (The sums run over K in the same order for every width.) A forward call of 128
-    // and 900 samples takes 87 and 101 us so, 99 and 113 with tiles of 128 columns throughout, 194 and 193
-    // with 256 columns over all 4,096 rows.
+    // A forward GEMM over M rows, with the narrowest tile whose CTAs still are one wave (all resident at
+    // once), else the widest: over few rows the pass is a chain of five launches that leave most SMs idle,
+    // and narrower tiles shorten each CTA's copies and epilogue. (The sums run over K in the same order for
+    // every width.) A forward call of 128 and 900 samples takes 80 and 94 us so, 194 and 193 with 256
+    // columns over all 4,096 rows. On 148 SMs, here / with the narrower tile kept a step beyond one wave:
+    // the output layer's 64 columns past 3 row tiles 84 / 91 us and its 128 past 6 the same (93); the
+    // hidden layers' 64 past 9 row tiles 105 / 124 and their 128 past 18 149 / 169.
     template <class Epi>
     cudaError_t mm_rows(const bf16 *A, const bf16 *B, int M, int N, int K, Epi epi) {
         const int rows_m = M / gemm::kBM;

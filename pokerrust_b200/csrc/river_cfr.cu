@@ -996,12 +996,15 @@ __global__ void __launch_bounds__(kFinThreads)
 }
 
 // CTAs per root. One CTA takes a root's 48 river cards one after the other, so few roots leave most
-// of the chip idle; more CTAs per root repeat its set-up and, in CFR passes, pass every card's bucket
-// sums through memory. The estimate counts waves of one CTA per SM, in units of a river card's work
-// (8.2 us in single precision, about twice that in double): set-up 1, handing a card's sums over 0.4,
-// finish_kernel 5 (best responses, which have no bucket sums: 2). Measured on a pass pair (CFR of both
-// players), whole / split: 1 root 730 / 96 us, 20 roots 797 / 241, 74 roots 800 / 623; best responses in
-// double with host copies, 1 root 1207 / 143, 149 roots 3216 / 2362.
+// of the chip idle; more CTAs per root repeat its set-up and pass every card's values and (in CFR passes)
+// bucket sums through memory. The estimate counts waves of one CTA per SM, in units of a river card's work
+// (8.2 us in a CFR pass, 6.7 in a best response, 14 in double): set-up 1, handing a card's sums over 0.4,
+// finish_kernel 5 (15 us over 1 root, 30 over 20, 55 over 74, from cold caches), 2 where there are no bucket
+// sums. On 148 SMs that splits CFR passes over 1-74 and 149-172 roots, best responses over 1-111 and
+// 149-240. Whole / split, passes alone on the device: a pair of CFR passes over 1 root 794 / 70 us, 20 roots
+// 800 / 229, 74 roots 804 / 638, 149 roots 1541 / 1424, 172 roots 1566 / 1495; a best response over 1 root
+// 328 / 21 us, 75 roots 328 / 241, 149 roots 634 / 440, 240 roots 645 / 603, in double 682 / 33, 687 / 486,
+// 1270 / 851 and 1342 / 1203.
 int pick_splits(int n, int sms, bool cfr) {
     if (n > kMaxSplitRoots) return 1;
     int best = 1;
