@@ -35,9 +35,9 @@ def test_many_builders_hold_one_pool():
     for b in builders:
         b.evaluate_device(tables, 0, False, d_in.data_ptr(), d_out.data_ptr())
     used = free - held()
-    # a pass over 70 roots takes more than 64 MB, the pool keeps 256 MB at most (64 MB to spare for the
-    # kernels, loaded on first use)
-    assert 64 << 20 < used <= 320 << 20, used >> 20
+    assert all(b.splits > 1 for b in builders)
+    # the pool keeps 256 MB at most (64 MB to spare for the kernels, loaded on first use)
+    assert used <= 320 << 20, used >> 20
     for b in builders:
         b.close()
     assert held() >= free
